@@ -26,6 +26,7 @@
 #include "common.h"
 #include "host_scene.h"
 #include "kernels.h"
+#include "mesh_upload.h"
 
 using namespace asuna;
 
@@ -35,13 +36,14 @@ namespace {
 
 constexpr uint64_t kBytesPerPath = 2 * 32 + 16 + 4 + 48 + 48 + 16 + 4 * kNumShadeClasses;
 
+// Device copy of an array (room for it where `host` is null), owned by the scene.
 template <class T>
 int devUpload(asuna_scene* s, const T* host, size_t n, const T** out) {
   void* p = nullptr;
   size_t bytes = std::max<size_t>(n * sizeof(T), 16);
   ASUNA_CUDA_TRY(cudaMalloc(&p, bytes));
   s->allocs.push_back(p);
-  if (n) ASUNA_CUDA_TRY(cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice));
+  if (n && host) ASUNA_CUDA_TRY(cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice));
   s->stats.device_bytes += bytes;
   *out = static_cast<const T*>(p);
   return ASUNA_OK;
@@ -336,7 +338,15 @@ int asuna_ctx_set_path_budget(asuna_ctx* c, uint64_t bytes) {
 int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** out) {
   clearError();
   if (!c || !d || !out) return fail(ASUNA_ERR_INVALID, "asuna_scene_create: null argument");
-  int rc = validateSceneDesc(d);
+  // Meshes are packed on the device from this many triangles on (scene
+  // creation 30.8 -> 21.3 ms at 2M triangles, 205 -> 103 ms at 21M); below,
+  // the host packs them in less time than the extra copies and launches take
+  // (both ways within 0.1 ms of each other at 10,000 triangles).
+  constexpr uint32_t kDevicePackTris = 4096;
+  uint64_t allTris = 0;
+  for (uint32_t m = 0; d->meshes && m < d->num_meshes; ++m) allTris += d->meshes[m].num_triangles;
+  const bool devicePack = allTris >= kDevicePackTris;
+  int rc = validateSceneDesc(d, !devicePack);
   if (rc) return rc;
   ASUNA_CUDA_TRY(cudaSetDevice(c->device));
   auto t0 = std::chrono::steady_clock::now();
@@ -355,7 +365,20 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
   if (triBase[nm] > kMaxLeafFirst) return fail(ASUNA_ERR_UNSUPPORTED, "scene has more than 2^28 triangles");
   // shading data first: the device build reads positions and indices from them
   SceneDev& v = s->view;
-  {
+  if (devicePack) {
+    VtxDev* dv = nullptr;
+    uint4* di = nullptr;
+    if ((rc = devUpload<VtxDev>(s, nullptr, vtxBase[nm], &v.vtx)) || (rc = devUpload<uint4>(s, nullptr, triBase[nm], &v.idx)))
+      return rc;
+    dv = const_cast<VtxDev*>(v.vtx);
+    di = const_cast<uint4*>(v.idx);
+    uint32_t bad = 0;
+    if ((rc = uploadMeshes(d, triBase, vtxBase, dv, di, c->stream, bad))) return rc;
+    if (bad) {  // (the host check names the mesh and the index)
+      rc = validateSceneDesc(d);
+      return rc ? rc : fail(ASUNA_ERR_INVALID, "%u triangles with an index out of range", bad);
+    }
+  } else {
     std::vector<VtxDev> vtx(vtxBase[nm]);
     std::vector<uint4> idx(triBase[nm]);
     for (uint32_t m = 0; m < nm; ++m) {

@@ -46,7 +46,7 @@ int fail(int code, const char* fmt, ...) {
 void clearError() { gLastError.clear(); }
 
 // ---- scene validation ---------------------------------------------------------
-int validateSceneDesc(const asuna_scene_desc* d) {
+int validateSceneDesc(const asuna_scene_desc* d, bool indices) {
   if (d->num_meshes && !d->meshes) return fail(ASUNA_ERR_INVALID, "meshes is NULL");
   if (d->num_instances && !d->instances) return fail(ASUNA_ERR_INVALID, "instances is NULL");
   if (d->num_materials && !d->materials) return fail(ASUNA_ERR_INVALID, "materials is NULL");
@@ -55,7 +55,7 @@ int validateSceneDesc(const asuna_scene_desc* d) {
     const asuna_mesh_desc& md = d->meshes[m];
     if (md.num_triangles && (!md.indices || !md.vertices))
       return fail(ASUNA_ERR_INVALID, "mesh %u: NULL vertex or index array", m);
-    for (uint64_t i = 0; i < uint64_t(md.num_triangles) * 3; ++i)
+    for (uint64_t i = 0; indices && i < uint64_t(md.num_triangles) * 3; ++i)
       if (md.indices[i] >= md.num_vertices)
         return fail(ASUNA_ERR_INVALID, "mesh %u: index %u out of range (%u vertices)", m, md.indices[i],
                     md.num_vertices);

@@ -10,7 +10,8 @@
 
 namespace asuna {
 
-int validateSceneDesc(const asuna_scene_desc* d);
+// `indices`: also that every index lies within its mesh (a pass over all of them)
+int validateSceneDesc(const asuna_scene_desc* d, bool indices = true);
 // world->object of an object->world 3x4 (row-major): double inverse, rounded once.
 void invert3x4(const float* m, float* out);
 
