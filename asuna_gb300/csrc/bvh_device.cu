@@ -4,11 +4,12 @@
 // (src/pipeline/pipeline_raytrace.cpp:107-147) with the same binned
 // surface-area-heuristic algorithm as the host builder (bvh_build.cpp): 32
 // bins per axis over the centroid bounds, cost 1 + (A_L N_L + A_R N_R) / A,
-// leaves of at most 4 triangles made where the SAH prefers them, index
+// leaves of at most 3 triangles made where the SAH prefers them, index
 // halving where all centroids coincide or past depth 40, child boxes widened
-// by a relative 2^-20.  The output is the traversal's layout: 64-byte
-// BvhNode (child boxes + refs), leaves as (first, count) ranges of 48-byte
-// TriDev records in leaf order.  Every mesh is built at once.
+// by a relative 2^-20.  The output is 64-byte BvhNode (child boxes + refs)
+// with leaves as (first, count) ranges of 48-byte TriDev records in leaf
+// order; bvh_wide.cu makes the traversal's nodes from it.  Every mesh is
+// built at once.
 //
 // Two phases:
 //  * large tasks (more than kSmallTask primitives) level by level: blocks
@@ -44,7 +45,7 @@ constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 constexpr uint32_t kSmallTask = 512;
 constexpr uint32_t kChunk = 4096;       // primitives per block in the large-task kernels
 constexpr uint32_t kMedianDepth = 40;   // past this depth: halve by index (depth stays bounded)
-constexpr int kMaxLeaf = 4;
+constexpr int kMaxLeaf = int(kWideLeaf);
 constexpr int kWarpStack = 60;          // pending subtasks of one warp's depth-first build
 constexpr uint32_t kNodeChunk = 16;  // (buildWarp takes up to 16 at once)
 constexpr int kSmallWarps = 4;          // warps per block in the small-task kernel

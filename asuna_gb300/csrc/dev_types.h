@@ -13,12 +13,10 @@
 namespace asuna {
 
 // ---- acceleration structure -------------------------------------------------
-// Binary BVH node, 64 B: the two child boxes, then the child references.
-// ref >= 0: inner node index; ref < 0: leaf, decoded by leafFirst/leafCount
-// (BLAS: first triangle, count <= 8; TLAS: instance).  The planes are laid
-// out in (x, y) pairs and a z quad, so the traversal computes the six slab
-// distances of a child with three packed two-lane operations against the
-// ray's (o.x, o.y) / (o.z, o.z) pairs.
+// Binary BVH node of the builders, 64 B: the two child boxes, then the child
+// references.  ref >= 0: inner node index; ref < 0: leaf, decoded by
+// leafFirst/leafCount (BLAS: first triangle, count <= kWideLeaf; TLAS:
+// instance).  The traversal reads WideNode, which is made from it.
 struct __align__(16) BvhNode {
   float4 xy[2];  // child c: lo.x, lo.y, hi.x, hi.y
   float4 zs;     // c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z
@@ -45,6 +43,25 @@ inline __host__ __device__ void nodeGetBox(const BvhNode& n, int c, float* lo, f
   hi[2] = z[2 * c + 1];
 }
 
+// 8-wide BVH node, 80 B (bvh_wide.cu makes it, trace.cu reads it): child
+// boxes as 8-bit offsets in a per-node frame, plane = p + q 2^e per axis.
+//   w[0]  p.xyz (floats); bytes: the axes' exponents e + kWideExpBias, then
+//         the mask of inner children
+//   w[1]  first inner child (the others follow in slot order); first leaf
+//         record (triangle, or index into the instance list); eight bytes,
+//         one per child: a leaf's record count << 5 | offset, else 0
+//   w[2]  lo.x of children 0-3, 4-7; lo.y likewise
+//   w[3]  lo.z; hi.x      w[4]  hi.y; hi.z
+// An empty slot is neither inner nor a leaf, and its box is inside out.
+struct __align__(16) WideNode {
+  uint4 w[5];
+};
+static_assert(sizeof(WideNode) == 80, "WideNode is 80 bytes");
+constexpr uint32_t kWideLeaf = 3;           // triangles of one leaf at most (8 leaves: offsets below 24)
+constexpr int kWideExpBias = 127 + 15;      // the traversal wants the float 2^(e + 15)
+constexpr int kWideMaxExp = 254 - kWideExpBias;
+constexpr float kWideFar = 1e34f;           // box planes beyond this (or NaN) are moved here
+
 constexpr int kMaxLeafTris = 8;
 constexpr int32_t kStackSentinel = INT32_MIN;  // "leave the BLAS" marker
 inline __host__ __device__ int32_t encodeLeaf(uint32_t first, uint32_t count) {
@@ -54,7 +71,7 @@ inline __host__ __device__ uint32_t leafFirst(int32_t ref) { return uint32_t(~re
 inline __host__ __device__ uint32_t leafCount(int32_t ref) { return (uint32_t(~ref) & 7u) + 1u; }
 constexpr uint32_t kMaxLeafFirst = (1u << 28) - 1u;
 
-// Leaf triangle in BVH order, 48 B: object-space vertices; v0.w holds the
+// Leaf triangle in leaf order, 48 B: object-space vertices; v0.w holds the
 // mesh-local primitive id (float bits).
 struct __align__(16) TriDev {
   float4 v0, v1, v2;
@@ -66,19 +83,23 @@ struct __align__(16) VtxDev {
   float4 nv;
 };
 
-// Instance record, 128 B.
-struct __align__(16) InstDev {
+// Instance record, 160 B; the traversal reads the first 32-byte sector before
+// it enters an instance.
+struct __align__(32) InstDev {
+  float boxLo[3];     // world box, as widened for the top level's leaf
+  int32_t blasRoot;   // root node of the mesh BLAS (-1: empty mesh)
+  float boxHi[3];
+  uint32_t rootLeaves;  // a root with leaves only, at most kWideLeaf triangles in all: its leaf slots; else 0
   float4 w2o[3];  // world -> object rows (double inverse rounded once)
   float4 o2w[3];  // object -> world rows (as given)
-  int32_t blasRoot;  // inner-node index of the mesh BLAS (-1: empty mesh)
   uint32_t vtxBase;  // first vertex of the mesh in the vertex arrays
   uint32_t idxBase;  // first triangle of the mesh in the index array
   int32_t matId;     // material (-1 for emitters)
   int32_t lightId;   // >= 0: emitter instance
   uint32_t matType;
-  uint32_t pad[2];
+  uint32_t pad[3];
 };
-static_assert(sizeof(InstDev) == 128, "InstDev is 128 bytes");
+static_assert(sizeof(InstDev) == 160, "InstDev is 160 bytes");
 
 // Packed material, 96 B: (diffuse.xyz, type bits), (alpha.x, alpha.y, ior,
 // fdrInt), (radiance.xyz, 0), (radiance_factor.xyz, 0); an emissive material
@@ -108,8 +129,9 @@ struct __align__(16) LightDev {
 
 // Device view of one uploaded scene.
 struct SceneDev {
-  const BvhNode* nodes;  // all BLAS nodes, then the TLAS nodes
+  const WideNode* nodes;  // the roots (every mesh's, then the top level's), then all other nodes
   const TriDev* tris;
+  const uint32_t* instIds;  // instances in the top level's leaf order
   const VtxDev* vtx;
   const uint4* idx;  // mesh-local vertex indices (x, y, z), w unused
   const InstDev* inst;

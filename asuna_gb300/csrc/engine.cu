@@ -23,6 +23,7 @@
 
 #include "bvh_build.h"
 #include "bvh_device.h"
+#include "bvh_wide.h"
 #include "common.h"
 #include "host_scene.h"
 #include "kernels.h"
@@ -397,7 +398,14 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
   // ---- bottom level: one BVH per mesh, on the device (default) or host threads ----
   const bool onDevice = c->bvhBuild == 0;
   std::vector<BvhBuildOut> blas(onDevice ? 0 : nm);
-  DeviceBlas dblas;
+  DeviceBlas dblas;  // binary trees and their triangles: dropped once the wide nodes are made
+  struct DropBinary {
+    DeviceBlas& d;
+    ~DropBinary() {
+      cudaFree(d.nodes);
+      cudaFree(d.tris);
+    }
+  } dropBinary{dblas};
   std::vector<BvhNode> nodes;
   std::vector<TriDev> tris;
   std::vector<int32_t> rootIndex(nm, -1);
@@ -406,14 +414,6 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
   const uint32_t extraNodes = 2 * d->num_instances + 4;
   if (onDevice) {
     rc = buildBlasDevice(v.vtx, v.idx, triBase, vtxBase, extraNodes, c->stream, dblas);
-    if (dblas.nodes) {
-      s->allocs.push_back(dblas.nodes);
-      s->stats.device_bytes += uint64_t(dblas.nodeCapacity) * sizeof(BvhNode);
-    }
-    if (dblas.tris) {
-      s->allocs.push_back(dblas.tris);
-      s->stats.device_bytes += uint64_t(std::max<uint32_t>(triBase[nm], 1)) * sizeof(TriDev);
-    }
     if (rc) return rc;
     blasNodes = dblas.nodeCount;
     blasDepth = dblas.maxDepth;
@@ -444,7 +444,7 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
                 cen[3 * i + k] = 0.5f * (boxes[i].lo[k] + boxes[i].hi[k]);
               }
             }
-            okMesh[m] = buildBvh(boxes, cen, 4, triBase[m], blas[m]) ? 1 : 0;
+            okMesh[m] = buildBvh(boxes, cen, int(kWideLeaf), triBase[m], blas[m]) ? 1 : 0;
           }
         });
       for (auto& t : th) t.join();
@@ -485,6 +485,13 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
       }
     }
   }
+  // wide node k is the root of the k-th mesh that has triangles
+  std::vector<int32_t> wideRoots, wideRoot(nm, -1);
+  for (uint32_t m = 0; m < nm; ++m)
+    if (rootIndex[m] >= 0) {
+      wideRoot[m] = int32_t(wideRoots.size());
+      wideRoots.push_back(rootIndex[m]);
+    }
   // ---- instances + top level ----
   const uint32_t ni = d->num_instances;
   std::vector<InstDev> inst(ni);
@@ -504,7 +511,7 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
     }
     const uint32_t m = id.mesh_id;
     const bool empty = d->meshes[m].num_triangles == 0;
-    I.blasRoot = empty ? -1 : rootIndex[m];
+    I.blasRoot = empty ? -1 : wideRoot[m];
     I.vtxBase = vtxBase[m];
     I.idxBase = triBase[m];
     I.matId = id.light_id >= 0 ? -1 : id.material_id;
@@ -537,6 +544,11 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
         wb.lo[k] = std::min(wb.lo[k], std::nextafter(float(v), -INFINITY));
         wb.hi[k] = std::max(wb.hi[k], std::nextafter(float(v), INFINITY));
       }
+    }
+    for (int k = 0; k < 3; ++k) {  // as widened in the top level's leaf
+      const float e = std::max(std::fabs(wb.lo[k]), std::fabs(wb.hi[k])) * 9.5367431640625e-07f + 1e-30f;
+      I.boxLo[k] = wb.lo[k] - e;
+      I.boxHi[k] = wb.hi[k] + e;
     }
     iboxes.push_back(wb);
     for (int k = 0; k < 3; ++k) icen.push_back(0.5f * (wb.lo[k] + wb.hi[k]));
@@ -653,18 +665,35 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
     asuna_envmap_tables(ew, eh, d->envmap.rgba, reinterpret_cast<float*>(marg.data()),
                         reinterpret_cast<float*>(cond.data()));
   }
+  // ---- binary trees of both levels -> wide nodes ----
   if (onDevice) {
     // the top level goes after the device-built bottom levels
-    v.nodes = dblas.nodes;
-    v.tris = dblas.tris;
     if (!tlasNodes.empty())
-      ASUNA_CUDA_TRY(cudaMemcpy(dblas.nodes + tlasBase, tlasNodes.data(), tlasNodes.size() * sizeof(BvhNode),
-                                cudaMemcpyHostToDevice));
+      ASUNA_CUDA_TRY(cudaMemcpyAsync(dblas.nodes + tlasBase, tlasNodes.data(), tlasNodes.size() * sizeof(BvhNode),
+                                     cudaMemcpyHostToDevice, c->stream));
   } else {
     nodes.insert(nodes.end(), tlasNodes.begin(), tlasNodes.end());
-    if ((rc = devUpload(s, nodes.data(), nodes.size(), &v.nodes)) || (rc = devUpload(s, tris.data(), tris.size(), &v.tris)))
-      return rc;
+    ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dblas.nodes), nodes.size() * sizeof(BvhNode)));
+    ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dblas.tris), std::max<size_t>(tris.size(), 1) * sizeof(TriDev)));
+    ASUNA_CUDA_TRY(cudaMemcpyAsync(dblas.nodes, nodes.data(), nodes.size() * sizeof(BvhNode), cudaMemcpyHostToDevice,
+                                   c->stream));
+    if (!tris.empty())
+      ASUNA_CUDA_TRY(cudaMemcpyAsync(dblas.tris, tris.data(), tris.size() * sizeof(TriDev), cudaMemcpyHostToDevice,
+                                     c->stream));
   }
+  wideRoots.push_back(int32_t(tlasBase));
+  WideBvh wide;
+  rc = buildWide(dblas.nodes, uint32_t(tlasBase + tlasNodes.size()), dblas.tris, triBase[nm], uint32_t(ids.size()),
+                 wideRoots, std::max(tlas.maxDepth, blasDepth), c->stream, wide);
+  for (void* p : {static_cast<void*>(wide.nodes), static_cast<void*>(wide.tris)})
+    if (p) s->allocs.push_back(p);
+  if (rc) return rc;
+  s->stats.device_bytes += wide.bytes;
+  for (InstDev& I : inst)
+    if (I.blasRoot >= 0) I.rootLeaves = wide.rootLeaves[size_t(I.blasRoot)];
+  v.nodes = wide.nodes;
+  v.tris = wide.tris;
+  v.instIds = wide.instIds;
   if ((rc = devUpload(s, inst.data(), inst.size(), &v.inst)) ||
       (rc = devUpload(s, mats.data(), mats.size(), &v.mats)) ||
       (rc = devUpload(s, lights.data(), lights.size(), &v.lights)) ||
@@ -673,7 +702,7 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
       (rc = devUpload(s, texels.data(), texels.size(), &v.texels)) ||
       (rc = devUpload(s, texInfo.data(), texInfo.size(), &v.texInfo)))
     return rc;
-  v.tlasRoot = int32_t(tlasBase);
+  v.tlasRoot = int32_t(wideRoots.size() - 1);
   std::memset(&v.sky, 0, sizeof(v.sky));
   if (d->sun_and_sky && d->sun_and_sky->in_use == 1) v.sky = *d->sun_and_sky;
   v.envW = int32_t(ew);

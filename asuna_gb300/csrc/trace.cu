@@ -8,16 +8,28 @@
 // (src/pipeline/pipeline_raytrace.cpp:132).
 //
 // Persistent warps refill their idle lanes from the queue (one atomic per
-// refill and warp); each thread walks TLAS -> BLAS with a per-thread stack
-// in shared memory (entry k of thread t at sstack[k * TB + t], bank-conflict
-// free) that spills into thread-local memory past its shared part.  Node and
-// triangle records are read with 128-bit read-only loads; the slab distances
-// of a node are computed with packed two-lane (f32x2) arithmetic.  The ray is
-// moved into object space and tested against triangles with the watertight
-// algorithm of Woop, Benthin and Wald (JCGT 2013) using explicitly rounded
-// operations, so the hits equal the CPU oracle's bit for bit; box tests use
-// (lo - o) * (1/d) with the far distance widened by 2^-20, which keeps them
-// conservative.
+// refill and warp); each thread walks the top level, then an instance's
+// bottom level, over 8-wide nodes of 80 bytes (bvh_wide.cu).  A node step
+// tests eight child boxes at once: the 8-bit planes become floats by byte
+// permutation (1 + q 2^-15) and the distances are one packed fused
+// multiply-add per plane pair.  What bounds the kernel is the chain of
+// dependent node fetches of a ray and the lanes that idle along: the wide
+// node makes that chain 2.8 times shorter than a binary one's.  On the
+// 21M-triangle benchmark scene (1920x1080, 8 frames, depth 12; ms per render):
+// closest hits 14.97 -> 10.06, occlusion 7.47 -> 3.89, nodes per ray
+// 24.4 -> 8.9; the issue slots are 73% busy with 14 of 32 lanes active.
+// The ray is moved into object space and tested against triangles with the
+// watertight algorithm of Woop, Benthin and Wald (JCGT 2013) using explicitly
+// rounded operations, so the hits equal the CPU oracle's bit for bit: they
+// depend on the triangle tests alone, not on the tree.
+//
+// The box tests are conservative.  With cell = 2^e, plane = p + q cell and
+// c = fl(fl(p - o) inv), a plane distance is fma(1 + q 2^-15, s, c - s) with
+// s = 2^15 cell inv.  Its error has a part relative to the distance itself
+// (the subtraction, the reciprocal, the products: under 2^-21 of it) and a
+// part of the frame: 2^-9 cell from rounding c - s, 2^-14 cell from the
+// cancellation between c and the offset.  The far distance is widened by
+// 2^-20, and every child box was quantised with 2^-5 cell to spare.
 #include <cuda_runtime.h>
 
 #include "kernels.h"
@@ -116,9 +128,8 @@ __device__ __forceinline__ float3 safeInv(float3 d) {
 }
 
 // Packed pairs of IEEE single-precision values in one 64-bit register pair:
-// the f32x2 add / mul of sm_100 and later issue as one instruction and round
-// each lane to nearest, like the scalar operations they replace, so the slab
-// distances are bit-identical to (plane - o) * (1/d) computed one by one.
+// the f32x2 fma of sm_100 and later issues as one instruction and rounds each
+// lane to nearest.
 typedef unsigned long long F2;
 __device__ __forceinline__ F2 pack2(float a, float b) {
   F2 r;
@@ -128,12 +139,15 @@ __device__ __forceinline__ F2 pack2(float a, float b) {
 __device__ __forceinline__ void unpack2(F2 p, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
 }
-// (planes - o) * inv, lane by lane; returns the two distances
-__device__ __forceinline__ void slab2(F2 planes, F2 o, F2 inv, float& t0, float& t1) {
-  F2 d, t;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(planes), "l"(o));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(d), "l"(inv));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t));
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// byte j of w as the float 1 + q 2^-15
+template <int J>
+__device__ __forceinline__ float planeOf(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604 | (J << 4)));
 }
 
 __device__ __forceinline__ void xformRay(const float4* w, float3 o, float3 d, float3& oo, float3& dd) {
@@ -147,42 +161,42 @@ __device__ __forceinline__ void xformRay(const float4* w, float3 o, float3 d, fl
 }
 
 constexpr float kFarScale = 1.00000095367431640625f;  // 1 + 2^-20
-constexpr int32_t kDone = INT32_MIN + 1;               // stack empty: traversal over
-constexpr int32_t kNoLeaf = INT32_MIN + 2;             // no postponed leaf
-constexpr uint32_t kTraceSpinCap = 1u << 20;           // inner steps of one warp pass
+constexpr uint32_t kTriGroup = 0x80000000u;            // stack entry: a leaf group (else a node group)
+constexpr uint32_t kHits = 0xffu;
+constexpr uint32_t kTraceSpinCap = 1u << 20;           // node steps of one warp pass
 constexpr uint32_t kTraceRayCap = 1u << 16;            // leaves + transitions of one ray
+// Lanes (of 32) that must want a node step for the warp to go on with node
+// steps while others wait at a leaf or a transition (closest hits of the
+// benchmark scene: 13.3 ms per render with 1, 10.4 with 8, 10.1 with 12, 11.7
+// with 16 on an earlier state of the kernel).
+constexpr int kNodeLanes = 12;
 
-__device__ __forceinline__ bool isLeafRef(int32_t r) { return r < 0 && r != kStackSentinel && r != kDone; }
-
-struct HitOut {
-  float u, v;  // (the distance is the traversal's `best`)
-  uint32_t prim, inst;
-};
-
-// Traversal state of one ray (while-while traversal with postponed leaves,
-// after Aila and Laine, "Understanding the efficiency of ray traversal on
-// GPUs", HPG 2009).  innerStep() visits one inner node; a BLAS leaf met
-// there is postponed and, when `speculate`, the lane goes on visiting inner
-// nodes while other lanes of the warp still look for a leaf.  leafOrMove()
-// then tests the triangles of one leaf, or makes one TLAS/BLAS transition.
+// Traversal state of one ray.  A node group is a set of children of one node
+// that the ray's box tests kept: (index of the first inner child, inner-child
+// mask << 8 | children left); a leaf group likewise (node, leaf slots left).
+// nodeStep() takes the next child of the node group in octant order, leaves
+// the rest on the stack and tests that child's eight boxes; leafStep() tests
+// the triangles of one leaf; move() enters an instance or leaves it.
 //
-// The state is kept small (the kernel is bound by the latency of its node
-// fetches, so resident warps matter): the world-space ray is read again from
-// its source at the few instance transitions instead of being held, the
-// watertight test's axis permutation is packed into one word, the closest
-// distance is `best`, and the stack cap comes from the launch.
-template <int TB, int SHS>  // threads per block, stack entries in shared memory
+// The state is kept small (64 registers with the node's 20 words in flight):
+// the world-space ray is read again from its source at the few instance
+// transitions instead of being held, the watertight test's axis permutation
+// is packed into one word, a closer hit goes to memory at once and only its
+// distance is held, and tmin and the stack cap come from the source and the
+// launch.
+template <int TB, int SHS>  // threads per block, 8-byte stack entries in shared memory
 struct Trav {
-  F2 oxy, oz2;  // ray origin in the current space: (o.x, o.y), (o.z, o.z)
-  F2 ixy, iz2;  // inverse direction in the current space, likewise
+  float ox, oy, oz, ix, iy, iz;  // ray origin and inverse direction in the current space
   float Sx, Sy, Sz;  // watertight shear of the current space's direction
   uint32_t kxyz;     // its axis permutation, kx | ky << 2 | kz << 4
-  float tmin, best;
+  uint32_t pref;     // slots on the near side, one byte per axis
+  float best;  // tmax, then the closest hit's distance
   uint32_t curInst;
-  int sp;  // stack entries in use
-  int32_t ref, leaf;
-  bool found, inBlas;
-  HitOut h;
+  int sp;      // stack entries in use
+  int bottom;  // entries below the current instance's (0: in the top level)
+  uint32_t gBase, gMask;
+  uint32_t tNode, tMask;
+  bool found;
 
   __device__ __forceinline__ void setShear(const WT& w) {
     Sx = w.Sx;
@@ -201,34 +215,49 @@ struct Trav {
     return w;
   }
 
-  __device__ __forceinline__ void init(const SceneDev& S, float3 ro, float3 rd, float t0, float t1) {
+  __device__ __forceinline__ void init(const SceneDev& S, float3 ro, float3 rd, float tmax) {
     setSpace(ro, safeInv(rd));
-    tmin = t0;
-    best = t1;
+    best = tmax;
     curInst = 0;
     sp = 0;
-    ref = S.tlasRoot;
-    leaf = kNoLeaf;
+    bottom = 0;
+    enterTree(uint32_t(S.tlasRoot));
     found = false;
-    inBlas = false;
+  }
+  // the root as the only child of a node group
+  __device__ __forceinline__ void enterTree(uint32_t root) {
+    gBase = root;
+    gMask = 0x101u;
+    tMask = 0u;
   }
 
   __device__ __forceinline__ void setSpace(float3 o, float3 inv) {
-    oxy = pack2(o.x, o.y);
-    oz2 = pack2(o.z, o.z);
-    ixy = pack2(inv.x, inv.y);
-    iz2 = pack2(inv.z, inv.z);
+    ox = o.x;
+    oy = o.y;
+    oz = o.z;
+    ix = inv.x;
+    iy = inv.y;
+    iz = inv.z;
+    pref = (ix < 0.0f ? 0xAAu : 0x55u) | (iy < 0.0f ? 0xCC00u : 0x3300u) | (iz < 0.0f ? 0xF00000u : 0x0F0000u);
   }
-  __device__ __forceinline__ float3 origin() const {
-    float x, y, z, z2;
-    unpack2(oxy, x, y);
-    unpack2(oz2, z, z2);
-    return make_float3(x, y, z);
+
+  __device__ __forceinline__ bool hasNodes() const { return (gMask & kHits) != 0u; }
+  __device__ __forceinline__ bool idle() const { return !hasNodes() && tMask == 0u; }
+
+  // the slot to visit next: the near side first, axis by axis
+  __device__ __forceinline__ uint32_t pick(uint32_t hits) const {
+    uint32_t a = hits & (pref >> 16);
+    hits = a ? a : hits;
+    a = hits & (pref >> 8);
+    hits = a ? a : hits;
+    a = hits & pref;
+    hits = a ? a : hits;
+    return hits & (0u - hits);
   }
 
   // Stack: the first SHS entries in shared memory (stride TB: bank-conflict
   // free), deeper ones in thread-local memory.
-  __device__ __forceinline__ void push(int32_t* sh, int32_t* loc, int32_t v, int lim, bool& ovf) {
+  __device__ __forceinline__ void push(uint2* sh, uint2* loc, uint2 v, int lim, bool& ovf) {
     if (sp >= lim) {
       ovf = true;
       return;
@@ -239,146 +268,222 @@ struct Trav {
       loc[sp - SHS] = v;
     ++sp;
   }
-  __device__ __forceinline__ int32_t popOrDone(const int32_t* sh, const int32_t* loc) {
-    if (sp == 0) return kDone;
+  __device__ __forceinline__ uint2 top(const uint2* sh, const uint2* loc) {
     --sp;
     return sp < SHS ? sh[sp * TB] : loc[sp - SHS];
   }
-
-  template <bool COUNT>
-  __device__ __forceinline__ void innerStep(const SceneDev& S, int32_t* sh, int32_t* loc, int lim, uint32_t& nNodes,
-                                            bool& ovf) {
-    const BvhNode* n = S.nodes + ref;
-    // the 16-byte plane records as pairs: (lo.x, lo.y), (hi.x, hi.y) of
-    // each child; (lo.z, hi.z) of child 0, of child 1
-    const ulonglong2 c0 = __ldg(reinterpret_cast<const ulonglong2*>(&n->xy[0]));
-    const ulonglong2 c1 = __ldg(reinterpret_cast<const ulonglong2*>(&n->xy[1]));
-    const ulonglong2 zs = __ldg(reinterpret_cast<const ulonglong2*>(&n->zs));
-    const int4 rr = __ldg(&n->ref);
-    if (COUNT) ++nNodes;
-    float tx0, tx1, ty0, ty1, tz0, tz1, ux0, ux1, uy0, uy1, uz0, uz1;
-    slab2(c0.x, oxy, ixy, tx0, ty0);
-    slab2(c0.y, oxy, ixy, tx1, ty1);
-    slab2(zs.x, oz2, iz2, tz0, tz1);
-    slab2(c1.x, oxy, ixy, ux0, uy0);
-    slab2(c1.y, oxy, ixy, ux1, uy1);
-    slab2(zs.y, oz2, iz2, uz0, uz1);
-    const float a0 = fmax3(fminf(tx0, tx1), fminf(ty0, ty1), fmaxf(fminf(tz0, tz1), tmin));
-    const float a1 = fmin3(fmaxf(tx0, tx1), fmaxf(ty0, ty1), fminf(fmaxf(tz0, tz1), best)) * kFarScale;
-    const float b0 = fmax3(fminf(ux0, ux1), fminf(uy0, uy1), fmaxf(fminf(uz0, uz1), tmin));
-    const float b1 = fmin3(fmaxf(ux0, ux1), fmaxf(uy0, uy1), fminf(fmaxf(uz0, uz1), best)) * kFarScale;
-    const bool h0 = a0 <= a1, h1 = b0 <= b1;
-    if (h0 && h1) {
-      const bool swap = b0 < a0;
-      push(sh, loc, swap ? rr.x : rr.y, lim, ovf);
-      ref = swap ? rr.y : rr.x;
-    } else if (h0 || h1) {
-      ref = h0 ? rr.x : rr.y;
-    } else {
-      ref = popOrDone(sh, loc);
-    }
-    if (inBlas && leaf == kNoLeaf && isLeafRef(ref)) {
-      leaf = ref;  // postpone: test it together with the other lanes' leaves
-      ref = popOrDone(sh, loc);
+  // the next group of the current level, if there is one
+  __device__ __forceinline__ void next(const uint2* sh, const uint2* loc) {
+    if (sp > bottom) {
+      const uint2 e = top(sh, loc);
+      if (e.y & kTriGroup) {
+        tNode = e.x;
+        tMask = e.y & kHits;
+      } else {
+        gBase = e.x;
+        gMask = e.y;
+      }
     }
   }
 
-  // Returns true when the traversal is over.  `src.world(i, o, d)` gives
-  // ray i's world-space origin and direction again.
-  template <bool ANY, bool COUNT, class Src>
-  __device__ __forceinline__ bool leafOrMove(const SceneDev& S, const Src& src, uint32_t idx, int32_t* sh,
-                                             int32_t* loc, int lim, uint32_t& nTris, bool& ovf) {
-    int32_t L = kNoLeaf;
-    if (leaf != kNoLeaf) {
-      L = leaf;
-      leaf = kNoLeaf;
-    } else if (inBlas && isLeafRef(ref)) {
-      L = ref;
-      ref = popOrDone(sh, loc);
+  // Child J of four: shifts a 1 into `miss` where the ray misses its box.
+  // (the sign of tf (1 + 2^-20) - tn, one rounding; where an infinity makes
+  // it NaN the child counts as hit, which is conservative)
+  template <int J>
+  __device__ __forceinline__ void testChild(uint32_t& miss, float tmin, uint32_t nx, uint32_t fx, uint32_t ny,
+                                            uint32_t fy, uint32_t nz, uint32_t fz, F2 sx, F2 sy, F2 sz, F2 cx, F2 cy,
+                                            F2 cz) const {
+    float tnx, tfx, tny, tfy, tnz, tfz;
+    unpack2(fma2(pack2(planeOf<J>(nx), planeOf<J>(fx)), sx, cx), tnx, tfx);
+    unpack2(fma2(pack2(planeOf<J>(ny), planeOf<J>(fy)), sy, cy), tny, tfy);
+    unpack2(fma2(pack2(planeOf<J>(nz), planeOf<J>(fz)), sz, cz), tnz, tfz);
+    const float tn = fmaxf(fmax3(tnx, tny, tnz), tmin);
+    const float tf = fminf(fmin3(tfx, tfy, tfz), best);
+    miss = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, kFarScale, -tn)), miss, 1);
+  }
+
+  template <bool COUNT>
+  __device__ __forceinline__ void nodeStep(const SceneDev& S, float tmin, uint2* sh, uint2* loc, int lim, uint32_t& nNodes,
+                                           bool& ovf) {
+    const uint32_t bit = pick(gMask & kHits);
+    const uint32_t child = gBase + __popc((gMask >> 8) & (bit - 1u));
+    gMask ^= bit;
+    const uint4* n = S.nodes[child].w;
+    const uint4 n0 = __ldg(n), n1 = __ldg(n + 1), n2 = __ldg(n + 2), n3 = __ldg(n + 3), n4 = __ldg(n + 4);
+    if (hasNodes()) push(sh, loc, make_uint2(gBase, gMask), lim, ovf);
+    if (COUNT) ++nNodes;
+    const bool gx = ix < 0.0f, gy = iy < 0.0f, gz = iz < 0.0f;
+    const float sx = __uint_as_float((n0.w & 0xffu) << 23) * ix, sy = __uint_as_float((n0.w & 0xff00u) << 15) * iy,
+                sz = __uint_as_float((n0.w & 0xff0000u) << 7) * iz;
+    const float cx = __fmaf_rn(__uint_as_float(n0.x) - ox, ix, -sx), cy = __fmaf_rn(__uint_as_float(n0.y) - oy, iy, -sy),
+                cz = __fmaf_rn(__uint_as_float(n0.z) - oz, iz, -sz);
+    const F2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+    const F2 cx2 = pack2(cx, cx), cy2 = pack2(cy, cy), cz2 = pack2(cz, cz);
+    uint32_t miss = 0u;
+    {
+      const uint32_t nx = gx ? n3.w : n2.y, fx = gx ? n2.y : n3.w, ny = gy ? n4.y : n2.w, fy = gy ? n2.w : n4.y,
+                     nz = gz ? n4.w : n3.y, fz = gz ? n3.y : n4.w;
+      testChild<3>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<2>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<1>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<0>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
     }
-    if (L != kNoLeaf) {
-      const uint32_t first = leafFirst(L), cnt = leafCount(L);
-      const WT wt = shear();
-      const float3 o = origin();
-      for (uint32_t k = 0; k < cnt; ++k) {
-        const TriDev* tr = S.tris + first + k;
-        const float4 p0 = __ldg(&tr->v0), p1 = __ldg(&tr->v1), p2 = __ldg(&tr->v2);
-        if (COUNT) ++nTris;
-        float t, b1, b2;
-        if (wtTri(wt, o, p0, p1, p2, tmin, best, t, b1, b2)) {
-          if (ANY) {
-            found = true;
-            return true;
-          }
-          const uint32_t prim = __float_as_uint(p0.w);
-          // exact ties resolve to the lowest (instance, primitive), so the
-          // result does not depend on traversal order
-          if (!found || t < best || (curInst < h.inst || (curInst == h.inst && prim < h.prim))) {
-            found = true;
-            best = t;
-            h.u = b1;
-            h.v = b2;
-            h.prim = prim;
-            h.inst = curInst;
-          }
+    {
+      const uint32_t nx = gx ? n3.z : n2.x, fx = gx ? n2.x : n3.z, ny = gy ? n4.x : n2.z, fy = gy ? n2.z : n4.x,
+                     nz = gz ? n4.z : n3.x, fz = gz ? n3.x : n4.z;
+      testChild<3>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<2>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<1>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+      testChild<0>(miss, tmin, nx, fx, ny, fy, nz, fz, sx2, sy2, sz2, cx2, cy2, cz2);
+    }
+    const uint32_t hits = ~miss & kHits, inner = n0.w >> 24, leaves = hits & ~inner;
+    gBase = n1.x;
+    gMask = inner << 8 | (hits & inner);
+    if (leaves) {
+      // (a lane that walked on with a leaf group in hand keeps the older one below)
+      if (tMask) push(sh, loc, make_uint2(tNode, kTriGroup | tMask), lim, ovf);
+      tNode = child;
+      tMask = leaves;
+    }
+    if (idle()) next(sh, loc);
+  }
+
+  // The next leaf of the leaf group: its first record and their number.
+  __device__ __forceinline__ uint32_t takeLeaf(const SceneDev& S, uint32_t& count) {
+    const uint32_t bit = pick(tMask);
+    tMask ^= bit;
+    const WideNode* n = S.nodes + tNode;
+    const uint32_t m = __ldg(reinterpret_cast<const uint8_t*>(&n->w[1].z) + (31 - __clz(int(bit))));
+    count = m >> 5;
+    return __ldg(&n->w[1].y) + (m & 31u);
+  }
+
+  // Tests one leaf; true when an occlusion ray is done.
+  template <bool ANY, bool COUNT, class Src>
+  __device__ __forceinline__ bool leafStep(const SceneDev& S, Src& src, uint32_t idx, uint2* sh, uint2* loc,
+                                           uint32_t& nTris) {
+    uint32_t cnt;
+    const uint32_t first = takeLeaf(S, cnt);
+    const WT wt = shear();
+    const float3 o = make_float3(ox, oy, oz);
+    const float tmin = src.tmin(idx);
+    for (uint32_t k = 0; k < cnt; ++k) {
+      const TriDev* tr = S.tris + first + k;
+      const float4 p0 = __ldg(&tr->v0), p1 = __ldg(&tr->v1), p2 = __ldg(&tr->v2);
+      if (COUNT) ++nTris;
+      float t, b1, b2;
+      if (wtTri(wt, o, p0, p1, p2, tmin, best, t, b1, b2)) {
+        if (ANY) {
+          found = true;
+          return true;
+        }
+        const uint32_t prim = __float_as_uint(p0.w);
+        // exact ties resolve to the lowest (instance, primitive), so the
+        // result does not depend on traversal order
+        if (!found || t < best || src.later(idx, curInst, prim)) {
+          found = true;
+          best = t;
+          src.store(idx, t, b1, b2, prim, curInst);
         }
       }
-      return false;
     }
-    if (ref == kDone) return true;
-    if (ref == kStackSentinel) {
-      // leaving a BLAS: back to the world-space ray
-      inBlas = false;
+    if (idle()) next(sh, loc);
+    return false;
+  }
+
+  // Enters the next instance of a top-level leaf group whose box the ray
+  // meets, or leaves the current one.  True when the traversal is over.  `src.world(i, o, d)` gives ray
+  // i's world-space origin and direction again.
+  template <class Src>
+  __device__ __forceinline__ bool move(const SceneDev& S, const Src& src, uint32_t idx, uint2* sh, uint2* loc, int lim,
+                                       bool& ovf) {
+    if (bottom == 0) {
+      while (tMask) {
+        uint32_t cnt;
+        const uint32_t at = takeLeaf(S, cnt);
+        if (!cnt) continue;
+        const uint32_t inst = __ldg(&S.instIds[at]);
+        const InstDev* in = S.inst + inst;
+        // the instance's own box against the distance as it is now: the
+        // 8-bit box of the top level may be much larger (a cell is up to
+        // 1/128 of its node, which may span the scene) and was tested earlier
+        const float4 lo = __ldg(reinterpret_cast<const float4*>(in->boxLo)),
+                     hi = __ldg(reinterpret_cast<const float4*>(in->boxHi));
+        const float x0 = (lo.x - ox) * ix, x1 = (hi.x - ox) * ix, y0 = (lo.y - oy) * iy, y1 = (hi.y - oy) * iy,
+                    z0 = (lo.z - oz) * iz, z1 = (hi.z - oz) * iz;
+        const float tn = fmax3(fminf(x0, x1), fminf(y0, y1), fmaxf(fminf(z0, z1), src.tmin(idx)));
+        const float tf = fmin3(fmaxf(x0, x1), fmaxf(y0, y1), fminf(fmaxf(z0, z1), best)) * kFarScale;
+        if (!(tn <= tf)) continue;
+        if (sp + 2 > lim) {
+          ovf = true;
+          continue;
+        }
+        push(sh, loc, make_uint2(gBase, gMask), lim, ovf);
+        push(sh, loc, make_uint2(tNode, kTriGroup | tMask), lim, ovf);
+        bottom = sp;
+        curInst = inst;
+        float3 wo, wd, o, d;
+        src.world(idx, wo, wd);
+        xformRay(in->w2o, wo, wd, o, d);
+        setSpace(o, safeInv(d));
+        setShear(wtPre(d));
+        enterTree(__float_as_uint(lo.w));
+        const uint32_t leaves = __float_as_uint(hi.w);
+        if (leaves) {  // a handful of triangles: straight to them
+          tNode = gBase;
+          tMask = leaves;
+          gMask = 0u;
+        }
+        return false;
+      }
+    } else {
       float3 wo, wd;
       src.world(idx, wo, wd);
       setSpace(wo, safeInv(wd));
-      ref = popOrDone(sh, loc);
-      return false;
+      const uint2 t = top(sh, loc), g = top(sh, loc);
+      bottom = 0;
+      gBase = g.x;
+      gMask = g.y;
+      tNode = t.x;
+      tMask = t.y & kHits;
     }
-    // TLAS leaf: enter the instance's BLAS in object space
-    curInst = leafFirst(ref);
-    const InstDev* in = S.inst + curInst;
-    const int32_t root = __ldg(&in->blasRoot);
-    if (root >= 0 && sp < lim) {
-      float3 wo, wd, o, d;
-      src.world(idx, wo, wd);
-      xformRay(in->w2o, wo, wd, o, d);
-      setSpace(o, safeInv(d));
-      setShear(wtPre(d));
-      inBlas = true;
-      push(sh, loc, kStackSentinel, lim, ovf);
-      ref = root;
-      return false;
-    }
-    if (root >= 0) ovf = true;
-    ref = popOrDone(sh, loc);
-    return false;
+    if (idle()) next(sh, loc);
+    return idle();
   }
 };
 
 // Persistent warp over a ray source.  Lanes whose ray is finished take the
 // next rays of the source (one fetch per refill, per warp) while the other
-// lanes keep traversing.  Src supplies count, fetch(n) -> first index (called
-// by one lane), commit(first, n) (called by every lane), load(i, tr) and
-// finish(i, tr).
-template <bool ANY, bool COUNT, bool SPEC, int TB, int SHS, class Src>
-__device__ __forceinline__ void traceWarp(const SceneDev& S, Src& src, int32_t* sh, int32_t* loc, uint32_t refill,
-                                          int lim, uint32_t& nNodes, uint32_t& nTris, bool& ovf) {
+// lanes keep traversing.  Src supplies count, warps (that share it), fetch(n) -> first index (called
+// by one lane), commit(first, n) (called by every lane), load(i, tr),
+// tmin(i), world(i, o, d), store(i, hit), later(i, inst, prim) (the hit stored
+// last belongs to a later instance or primitive) and finish(i, found).
+template <bool ANY, bool COUNT, int TB, int SHS, class Src>
+__device__ __forceinline__ void traceWarp(const SceneDev& S, Src& src, uint2* sh, uint2* loc, uint32_t refill,
+                                          bool spec, int lim, uint32_t& nNodes, uint32_t& nTris, bool& ovf) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanesBelow = (1u << lane) - 1u;
+  // Lanes in use: a short queue is spread over all warps of the grid, so that
+  // fewer rays share (and serialise) a warp (a 320x180 preview's closest hits
+  // 0.65 -> 0.41 ms, a 1280x720 frame's 0.92 -> 0.72).
+  const uint32_t use = min(32u, max(1u, (src.count + src.warps - 1u) / src.warps));
+  const unsigned usable = 0xffffffffu >> (32u - use);
+  const int nodeLanes = int(use) * kNodeLanes / 32;
   bool active = false, drained = false;
   uint32_t idx = 0, events = 0;
   Trav<TB, SHS> tr;
+  tr.gMask = tr.tMask = 0u;
+  tr.bottom = 0;
   for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    if (idle && !drained && (uint32_t(__popc(idle)) >= refill || idle == 0xffffffffu)) {
+    const unsigned idle = __ballot_sync(0xffffffffu, !active) & usable;
+    if (idle && !drained && (uint32_t(__popc(idle)) >= refill || idle == usable)) {
       const int leader = __ffs(idle) - 1;
       uint32_t base = 0;
       if (int(lane) == leader) base = src.fetch(uint32_t(__popc(idle)));
       base = __shfl_sync(0xffffffffu, base, leader);
       src.commit(base, uint32_t(__popc(idle)));
       drained = base + uint32_t(__popc(idle)) >= src.count;
-      if (!active) {
+      if (idle >> lane & 1u) {
         const uint32_t r = base + uint32_t(__popc(idle & lanesBelow));
         if (r < src.count) {
           idx = r;
@@ -388,32 +493,48 @@ __device__ __forceinline__ void traceWarp(const SceneDev& S, Src& src, int32_t* 
         }
       }
     }
-    if (!__any_sync(0xffffffffu, active)) {
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    if (!act) {
       if (drained) break;
       continue;
     }
-    // inner nodes until every lane holds a leaf (or waits at a transition)
-    // (lanes without a leaf make progress every iteration, so the loop ends;
-    // with SPEC the others walk on speculatively meanwhile).  Both loops
-    // carry a bound far above any real traversal: past it the warp stops
-    // and reports the error instead of running on.
+    // Node steps while enough lanes want one.  Lanes with a leaf group in
+    // hand walk on when `spec` (and there is room for a second group on the
+    // stack).  A pass that stops early leaves lanes at a leaf or a
+    // transition, which go on below: some lane advances in every round.
+    // Both loops carry a bound far above any real traversal: past it the
+    // warp stops and reports the error instead of running on.
     uint32_t spin = 0;
     for (;;) {
-      const bool stepping = active && tr.ref >= 0;
-      const bool needy = stepping && tr.leaf == kNoLeaf;
-      if (!__any_sync(0xffffffffu, needy)) break;
+      const bool want = active && tr.hasNodes() && tr.tMask == 0u;
+      const unsigned wm = __ballot_sync(0xffffffffu, want);
+      if (wm == 0u || (__popc(wm) < nodeLanes && wm != act)) break;
       if (++spin > kTraceSpinCap) break;
-      if (SPEC ? stepping : needy) tr.template innerStep<COUNT>(S, sh, loc, lim, nNodes, ovf);
+      if (want || (spec && active && tr.hasNodes() && tr.bottom != 0 && tr.sp + 4 < lim))
+        tr.template nodeStep<COUNT>(S, src.tmin(idx), sh, loc, lim, nNodes, ovf);
     }
     if (spin > kTraceSpinCap) {
       ovf = true;
       break;
     }
-    if (active && (tr.template leafOrMove<ANY, COUNT>(S, src, idx, sh, loc, lim, nTris, ovf) ||
-                   ++events > kTraceRayCap)) {
-      if (events > kTraceRayCap) ovf = true;
+    bool done = false;
+    if (active && tr.bottom != 0 && tr.tMask != 0u) {
+      done = tr.template leafStep<ANY, COUNT>(S, src, idx, sh, loc, nTris);
+      ++events;
+    }
+    __syncwarp();
+    if (active && !done && (tr.bottom == 0 ? tr.tMask != 0u || tr.idle() : tr.idle())) {
+      done = tr.move(S, src, idx, sh, loc, lim, ovf);
+      ++events;
+    }
+    if (events > kTraceRayCap) {
+      ovf = true;
+      done = active;
+    }
+    if (done) {
       active = false;
-      src.finish(idx, tr);
+      events = 0;
+      src.finish(idx, tr.found);
     }
   }
 }
@@ -425,28 +546,33 @@ struct QueueSrc {
   const KParams* P;
   const float4 *rO, *rD;
   uint32_t* fetchCtr;
-  uint32_t count;
+  uint32_t count, warps;
   __device__ __forceinline__ uint32_t fetch(uint32_t n) { return atomicAdd(fetchCtr, n); }
   __device__ __forceinline__ void commit(uint32_t, uint32_t) {}
   template <class T>
   __device__ __forceinline__ void load(const SceneDev& S, uint32_t r, T& tr) {
     const float4 o4 = __ldg(&rO[r]);
     const float4 d4 = __ldg(&rD[r]);
-    if (ANY)
-      tr.init(S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), 0.0f, o4.w);
-    else
-      tr.init(S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), 0.00001f, 10000000000.0f);
+    tr.init(S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), ANY ? o4.w : 10000000000.0f);
   }
+  __device__ __forceinline__ float tmin(uint32_t) const { return ANY ? 0.0f : 0.00001f; }
   __device__ __forceinline__ void world(uint32_t r, float3& o, float3& d) const {
     const float4 o4 = __ldg(&rO[r]);
     const float4 d4 = __ldg(&rD[r]);
     o = make_float3(o4.x, o4.y, o4.z);
     d = make_float3(d4.x, d4.y, d4.z);
   }
-  template <class T>
-  __device__ __forceinline__ void finish(uint32_t i, const T& tr) {
+  __device__ __forceinline__ void store(uint32_t i, float t, float u, float v, uint32_t prim, uint32_t inst) {
+    W->hit[i] = make_float4(t, u, v, __uint_as_float(prim));
+    W->hitInst[i] = inst;
+  }
+  __device__ __forceinline__ bool later(uint32_t i, uint32_t inst, uint32_t prim) const {
+    const uint32_t h = W->hitInst[i];
+    return inst < h || (inst == h && prim < __float_as_uint(W->hit[i].w));
+  }
+  __device__ __forceinline__ void finish(uint32_t i, bool found) {
     if (ANY) {
-      if (!tr.found) {
+      if (!found) {
         const uint32_t p = __float_as_uint(__ldg(&rD[i].w));
         const float4 c = __ldg(&W->shC[i]);
         float4 r = W->rad[p];
@@ -456,10 +582,7 @@ struct QueueSrc {
         W->rad[p] = r;
         if (P->records) W->rec[p].y |= 1u << (P->depth - (W->path[p].info.y >> kPassShift) - 1u);
       }
-    } else if (tr.found) {
-      W->hit[i] = make_float4(tr.best, tr.h.u, tr.h.v, __uint_as_float(tr.h.prim));
-      W->hitInst[i] = tr.h.inst;
-    } else {
+    } else if (!found) {
       W->hit[i] = make_float4(-1.0f, 0.0f, 0.0f, 0.0f);
       W->hitInst[i] = 0xffffffffu;
     }
@@ -467,12 +590,12 @@ struct QueueSrc {
 };
 
 // TB: threads per block; MINB: resident blocks per SM the variant is
-// compiled for (its register cap); SHS: stack entries in shared memory
-template <bool ANY, bool COUNT, bool SPEC, int TB, int MINB, int SHS>
+// compiled for (its register cap); SHS: 8-byte stack entries in shared memory
+template <bool ANY, bool COUNT, int TB, int MINB, int SHS>
 __global__ void __launch_bounds__(TB, MINB) k_trace(KParams P) {
-  __shared__ int32_t sstack[SHS * TB];
-  int32_t lstack[kStackDepth - SHS];
-  int32_t* sh = sstack + threadIdx.x;
+  __shared__ uint2 sstack[SHS * TB];
+  uint2 lstack[kStackDepth - SHS];
+  uint2* sh = sstack + threadIdx.x;
   const WaveDev& W = P.W;
   const int cur = P.cur;
   uint32_t* countPtr = ANY ? &W.cnt->c[kCntShadow] : &W.cnt->c[kCntExtend0 + cur];
@@ -481,6 +604,7 @@ __global__ void __launch_bounds__(TB, MINB) k_trace(KParams P) {
   src.P = &P;
   src.fetchCtr = ANY ? &W.cnt->c[kCntFetchShadow] : &W.cnt->c[kCntFetchExtend];
   src.count = *countPtr;
+  src.warps = gridDim.x * (TB / 32);
   src.rO = ANY ? W.shO : W.rayO[cur];
   src.rD = ANY ? W.shD : W.rayD[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -499,7 +623,8 @@ __global__ void __launch_bounds__(TB, MINB) k_trace(KParams P) {
   // (the instrumented variant walks without speculation, so its node counts
   // are those of the ordered traversal)
   // (P.stackLimit is in [1, kStackDepth]: the host clamps it)
-  traceWarp<ANY, COUNT, SPEC, TB, SHS>(P.S, src, sh, lstack, P.refillLanes, P.stackLimit, nNodes, nTris, ovf);
+  traceWarp<ANY, COUNT, TB, SHS>(P.S, src, sh, lstack, P.refillLanes, !COUNT && P.speculate != 0, P.stackLimit, nNodes,
+                                 nTris, ovf);
   if (ovf) atomicAdd(&W.cnt->stackOverflow, 1ull);
   if (COUNT) {
     const unsigned lane = threadIdx.x & 31u;
@@ -523,25 +648,34 @@ struct ArraySrc {
   uint32_t* inst;
   uint32_t cursor, count;
   int anyHit;
+  static constexpr uint32_t warps = 1u;  // each warp has its own slice
   __device__ __forceinline__ uint32_t fetch(uint32_t) { return cursor; }
   // every lane of the warp advances its copy of the cursor alike
   __device__ __forceinline__ void commit(uint32_t base, uint32_t n) { cursor = base + n; }
   template <class T>
   __device__ __forceinline__ void load(const SceneDev& S, uint32_t r, T& tr) {
     const float4 o4 = o[r], d4 = d[r];
-    tr.init(S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), o4.w, d4.w);
+    tr.init(S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), d4.w);
   }
+  __device__ __forceinline__ float tmin(uint32_t r) const { return o[r].w; }
   __device__ __forceinline__ void world(uint32_t r, float3& wo, float3& wd) const {
     const float4 o4 = o[r], d4 = d[r];
     wo = make_float3(o4.x, o4.y, o4.z);
     wd = make_float3(d4.x, d4.y, d4.z);
   }
-  template <class T>
-  __device__ __forceinline__ void finish(uint32_t i, const T& tr) {
-    if (tr.found) {
-      hit[i] = anyHit ? make_float4(1.0f, 0.0f, 0.0f, 0.0f)
-                      : make_float4(tr.best, tr.h.u, tr.h.v, __uint_as_float(tr.h.prim));
-      inst[i] = anyHit ? 0u : tr.h.inst;
+  __device__ __forceinline__ void store(uint32_t i, float t, float u, float v, uint32_t prim, uint32_t in) {
+    hit[i] = make_float4(t, u, v, __uint_as_float(prim));
+    inst[i] = in;
+  }
+  __device__ __forceinline__ bool later(uint32_t i, uint32_t in, uint32_t prim) const {
+    return in < inst[i] || (in == inst[i] && prim < __float_as_uint(hit[i].w));
+  }
+  __device__ __forceinline__ void finish(uint32_t i, bool found) {
+    if (found) {
+      if (anyHit) {
+        hit[i] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+        inst[i] = 0u;
+      }
     } else {
       hit[i] = make_float4(-1.0f, 0.0f, 0.0f, 0.0f);
       inst[i] = 0xffffffffu;
@@ -551,9 +685,10 @@ struct ArraySrc {
 
 __global__ void __launch_bounds__(kTraceThreads) k_query(SceneDev S, const float4* o, const float4* d, uint32_t n,
                                                          int anyHit, float4* hit, uint32_t* inst) {
-  __shared__ int32_t sstack[kSharedStack * kTraceThreads];
-  int32_t lstack[kStackDepth - kSharedStack];
-  int32_t* sh = sstack + threadIdx.x;
+  constexpr int SHS = kSharedStack / 2;
+  __shared__ uint2 sstack[SHS * kTraceThreads];
+  uint2 lstack[kStackDepth - SHS];
+  uint2* sh = sstack + threadIdx.x;
   const uint32_t warps = gridDim.x * (blockDim.x / 32u);
   const uint32_t w = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
   const uint32_t per = (n + warps - 1) / warps;
@@ -563,11 +698,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_query(SceneDev S, const float
   uint32_t a = 0, b = 0;
   bool ovf = false;
   if (anyHit)
-    traceWarp<true, false, true, kTraceThreads, kSharedStack>(S, src, sh, lstack, kRefillLanes, kStackDepth, a, b,
-                                                              ovf);
+    traceWarp<true, false, kTraceThreads, SHS>(S, src, sh, lstack, kRefillLanes, true, kStackDepth, a, b, ovf);
   else
-    traceWarp<false, false, true, kTraceThreads, kSharedStack>(S, src, sh, lstack, kRefillLanes, kStackDepth, a, b,
-                                                               ovf);
+    traceWarp<false, false, kTraceThreads, SHS>(S, src, sh, lstack, kRefillLanes, true, kStackDepth, a, b, ovf);
 }
 
 }  // namespace
@@ -575,23 +708,16 @@ __global__ void __launch_bounds__(kTraceThreads) k_query(SceneDev S, const float
 namespace {
 // Kernel variants: threads per block (64, 128, 256) x resident warps per SM
 // (32, 40, 48: the occupancy class 8, 10, 12 of 128-thread blocks) x stack
-// entries in shared memory (16, 24, 32).
-template <bool ANY, int TB, int OCC, int SHS>
-void launchShape(const KParams& P, int grid, cudaStream_t s) {
-  constexpr int MINB = OCC * 128 / TB;
-  if (P.speculate)
-    k_trace<ANY, false, true, TB, MINB, SHS><<<grid, TB, 0, s>>>(P);
-  else
-    k_trace<ANY, false, false, TB, MINB, SHS><<<grid, TB, 0, s>>>(P);
-}
+// bytes in shared memory (16, 24, 32 words, two per entry).
 template <bool ANY, int TB, int OCC>
 void launchOcc(const KParams& P, int grid, cudaStream_t s) {
+  constexpr int MINB = OCC * 128 / TB;
   if (P.sharedStack >= 32)
-    launchShape<ANY, TB, OCC, 32>(P, grid, s);
+    k_trace<ANY, false, TB, MINB, 16><<<grid, TB, 0, s>>>(P);
   else if (P.sharedStack > 0 && P.sharedStack <= 16)
-    launchShape<ANY, TB, OCC, 16>(P, grid, s);
+    k_trace<ANY, false, TB, MINB, 8><<<grid, TB, 0, s>>>(P);
   else
-    launchShape<ANY, TB, OCC, 24>(P, grid, s);
+    k_trace<ANY, false, TB, MINB, 12><<<grid, TB, 0, s>>>(P);
 }
 template <bool ANY, int TB>
 void launchTb(const KParams& P, int grid, cudaStream_t s) {
@@ -605,7 +731,7 @@ void launchTb(const KParams& P, int grid, cudaStream_t s) {
 template <bool ANY>
 void launchTrace(const KParams& P, int grid, cudaStream_t s) {
   if (P.counters)
-    k_trace<ANY, true, false, kTraceThreads, kTraceMinBlocks, kSharedStack><<<grid, kTraceThreads, 0, s>>>(P);
+    k_trace<ANY, true, kTraceThreads, kTraceMinBlocks, kSharedStack / 2><<<grid, kTraceThreads, 0, s>>>(P);
   else if (P.blockThreads == 64)
     launchTb<ANY, 64>(P, grid, s);
   else if (P.blockThreads == 256)
@@ -616,13 +742,13 @@ void launchTrace(const KParams& P, int grid, cudaStream_t s) {
 template <int TB, int OCC, int SHS>
 int blocksOf() {
   int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trace<false, false, true, TB, OCC * 128 / TB, SHS>, TB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trace<false, false, TB, OCC * 128 / TB, SHS>, TB, 0);
   return n;
 }
 template <int TB, int OCC>
 int blocksOcc(int sharedStack) {
-  return sharedStack >= 32 ? blocksOf<TB, OCC, 32>()
-         : (sharedStack > 0 && sharedStack <= 16) ? blocksOf<TB, OCC, 16>() : blocksOf<TB, OCC, 24>();
+  return sharedStack >= 32 ? blocksOf<TB, OCC, 16>()
+         : (sharedStack > 0 && sharedStack <= 16) ? blocksOf<TB, OCC, 8>() : blocksOf<TB, OCC, 12>();
 }
 template <int TB>
 int blocksTb(int occupancy, int sharedStack) {
