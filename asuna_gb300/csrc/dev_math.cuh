@@ -251,8 +251,7 @@ __device__ __forceinline__ f3 uniformSampleSphere(f2 u) {
 }
 // sun_and_sky.glsl:405-533 (include/asuna_sunsky.h) in world direction L
 __device__ __noinline__ f3 evalSunSky(const SceneDev& S, f3 L) {
-  const asuna_sky::Params<float> p = asuna_sky::paramsOf<float>(S.sky);
-  const asuna_sky::V<float> r = asuna_sky::sunAndSky<float>(p, asuna_sky::V<float>{L.x, L.y, L.z});
+  const asuna_sky::V<float> r = asuna_sky::sunAndSky<float>(S.skyState, asuna_sky::V<float>{L.x, L.y, L.z});
   return f3{r.x, r.y, r.z};
 }
 // sample_light.glsl:84-95

@@ -9,6 +9,7 @@
 #include <vector_types.h>
 
 #include "../../include/asuna_rt.h"
+#include "../../include/asuna_sunsky.h"
 
 namespace asuna {
 
@@ -150,6 +151,7 @@ struct SceneDev {
   uint32_t classMask;  // shading classes some instance can reach (bit k = class k)
   uint32_t passThrough;  // 1: some material can pass rays through (opacity)
   asuna_sun_and_sky sky;  // in_use = 1: the sun & sky replaces the environment map
+  asuna_sky::SkyState<float> skyState;  // its direction-independent part
 };
 // Wavefront passes of a batch: one per bounce, plus the pass-through reserve.
 inline int wavefrontPasses(int maxDepth, const SceneDev& S) {

@@ -28,6 +28,9 @@ constexpr int kSharedStack = 24;     // of which in shared memory (the rest in l
 constexpr int kRefillLanes = 8;      // default idle lanes of a warp that trigger a queue fetch
 constexpr int kShadeMinBlocks = 3;   // resident 256-thread blocks per SM the shading kernel is compiled for
 
+// S.skyState of S.sky (evaluated on the device, with the shading kernels'
+// rounding; waits for the stream)
+int prepareSky(SceneDev& S, cudaStream_t s);
 void launchRaygen(const KParams& P, int grid, cudaStream_t s);
 void launchShade(const KParams& P, int grid, cudaStream_t s);
 // kernels launchShade issues for a scene's class mask (classify included)

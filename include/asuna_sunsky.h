@@ -185,26 +185,42 @@ ASUNA_SKY_FN V<R> sunColor(V<R> sd, R turbidity) {
   return out;
 }
 
-/* the Perez distribution term shared by sky_color_xyz and sky_luminance:
+/* The Perez distribution term shared by sky_color_xyz and sky_luminance:
  * ((1 + A e^{B / cos theta}) (1 + C e^{D gamma} + E cos^2 gamma)) /
- * ((1 + A e^{B}) (1 + C e^{D theta_s} + E cos^2 theta_s)) */
-ASUNA_SKY_FN R perez(R A, R B, R C, R D, R E, R cosTheta, R gamma, R cosGamma, R thetaSun, R cosThetaSun) {
-  return ((R(1) + A * m_exp(B / cosTheta)) * (R(1) + C * m_exp(D * gamma) + E * cosGamma * cosGamma)) /
-         ((R(1) + A * m_exp(B / R(1.0f))) * (R(1) + C * m_exp(D * thetaSun) + E * cosThetaSun * cosThetaSun));
+ * ((1 + A e^{B}) (1 + C e^{D theta_s} + E cos^2 theta_s)); the denominator
+ * depends on the sun and the turbidity only. */
+template <class R>
+struct Perez {
+  R A, B, C, D, E, den;
+};
+ASUNA_SKY_FN Perez<R> perezOf(R A, R B, R C, R D, R E, R thetaSun, R cosThetaSun) {
+  return Perez<R>{A, B, C, D, E,
+                  (R(1) + A * m_exp(B / R(1.0f))) *
+                      (R(1) + C * m_exp(D * thetaSun) + E * cosThetaSun * cosThetaSun)};
+}
+ASUNA_SKY_FN R perez(const Perez<R>& p, R cosTheta, R gamma, R cosGamma) {
+  return ((R(1) + p.A * m_exp(p.B / cosTheta)) * (R(1) + p.C * m_exp(p.D * gamma) + p.E * cosGamma * cosGamma)) /
+         p.den;
 }
 
-/* sun_and_sky.glsl:134-200: CIE XYZ of the sky in direction d */
-ASUNA_SKY_FN V<R> skyXYZ(V<R> d, V<R> sun, R T, R lum) {
-  R cg = vdot(sun, d);
-  if (cg > R(1.0f)) cg = R(2.0f) - cg;
-  const R gamma = m_acos(cg);
-  const R ct = d.z, cts = sun.z;
+/* What the sky's radiance in any direction needs of the sun direction `sun`
+ * and the turbidity T: sun_and_sky.glsl:134-245 without the direction. */
+template <class R>
+struct SkyConst {
+  V<R> sun;
+  R zx, zy, lum;  // zenith chromaticities and luminance
+  Perez<R> px, py, pl;
+};
+ASUNA_SKY_FN SkyConst<R> skyConst(V<R> sun, R T) {
+  SkyConst<R> k;
+  k.sun = sun;
+  const R cts = sun.z;
   const R ts = m_acos(cts);
   const R t2 = T * T, ts2 = ts * ts, ts3 = ts2 * ts;
-  const R zx = (R(0.001650f) * ts3 - R(0.003742f) * ts2 + R(0.002088f) * ts + R(0)) * t2 +
+  k.zx = (R(0.001650f) * ts3 - R(0.003742f) * ts2 + R(0.002088f) * ts + R(0)) * t2 +
                (R(-0.029028f) * ts3 + R(0.063773f) * ts2 - R(0.032020f) * ts + R(0.003948f)) * T +
                (R(0.116936f) * ts3 - R(0.211960f) * ts2 + R(0.060523f) * ts + R(0.258852f));
-  const R zy = (R(0.002759f) * ts3 - R(0.006105f) * ts2 + R(0.003162f) * ts + R(0)) * t2 +
+  k.zy = (R(0.002759f) * ts3 - R(0.006105f) * ts2 + R(0.003162f) * ts + R(0)) * t2 +
                (R(-0.042149f) * ts3 + R(0.089701f) * ts2 - R(0.041536f) * ts + R(0.005158f)) * T +
                (R(0.153467f) * ts3 - R(0.267568f) * ts2 + R(0.066698f) * ts + R(0.266881f));
   R A = R(-0.019257f) * T - (R(0.29f) - m_pow(cts, R(0.5f)) * R(0.09f));
@@ -212,42 +228,50 @@ ASUNA_SKY_FN V<R> skyXYZ(V<R> d, V<R> sun, R T, R lum) {
   R C = R(-0.000417f) * T + R(0.212479f);
   R D = R(-0.064097f) * T - R(0.898875f);
   R E = R(-0.003251f) * T + R(0.045178f);
-  R x = perez(A, B, C, D, E, ct, gamma, cg, ts, cts);
+  k.px = perezOf(A, B, C, D, E, ts, cts);
   A = R(-0.016698f) * T - R(0.260787f);
   B = R(-0.094958f) * T + R(0.009213f);
   C = R(-0.007928f) * T + R(0.210230f);
   D = R(-0.044050f) * T - R(1.653694f);
   E = R(-0.010922f) * T + R(0.052919f);
-  R y = perez(A, B, C, D, E, ct, gamma, cg, ts, cts);
+  k.py = perezOf(A, B, C, D, E, ts, cts);
+  // sky luminance, 202-227 and 229-236
+  A = R(0.178721f) * T - R(1.463037f);
+  B = R(-0.355402f) * T + R(0.427494f);
+  C = R(-0.022669f) * T + R(5.325056f);
+  D = R(0.120647f) * T - R(2.577052f);
+  E = R(-0.066967f) * T + R(0.370275f);
+  k.pl = perezOf(A, B, C, D, E, ts, cts);
+  const R chi = (R(4.0f) / R(9.0f) - T / R(120.0f)) * (kPi<R>() - R(2) * ts);
+  k.lum = R(1000.0f) * ((R(4.0453f) * T - R(4.9710f)) * m_tan(chi) - R(0.2155f) * T + R(2.4192f));
+  return k;
+}
+
+/* sun_and_sky.glsl:134-200: CIE XYZ of the sky in direction d */
+ASUNA_SKY_FN V<R> skyXYZ(const SkyConst<R>& k, V<R> d, R lum) {
+  R cg = vdot(k.sun, d);
+  if (cg > R(1.0f)) cg = R(2.0f) - cg;
+  const R gamma = m_acos(cg);
+  R x = perez(k.px, d.z, gamma, cg);
+  R y = perez(k.py, d.z, gamma, cg);
   const R sat = R(1.0f);
-  x = zx * ((x * sat) + (R(1.0f) - sat));
-  y = zy * ((y * sat) + (R(1.0f) - sat));
+  x = k.zx * ((x * sat) + (R(1.0f) - sat));
+  y = k.zy * ((y * sat) + (R(1.0f) - sat));
   return v3((x / y) * lum, lum, ((R(1.0f) - x - y) / y) * lum);
 }
 
 /* sun_and_sky.glsl:202-227: relative sky luminance (Perez, Y) */
-ASUNA_SKY_FN R skyLuminance(V<R> d, V<R> sun, R T) {
-  R cg = vdot(sun, d);
+ASUNA_SKY_FN R skyLuminance(const SkyConst<R>& k, V<R> d) {
+  R cg = vdot(k.sun, d);
   if (cg < R(0.0f)) cg = R(0.0f);
   if (cg > R(1.0f)) cg = R(2.0f) - cg;
-  const R gamma = m_acos(cg);
-  const R ct = d.z, cts = sun.z;
-  const R ts = m_acos(cts);
-  const R A = R(0.178721f) * T - R(1.463037f);
-  const R B = R(-0.355402f) * T + R(0.427494f);
-  const R C = R(-0.022669f) * T + R(5.325056f);
-  const R D = R(0.120647f) * T - R(2.577052f);
-  const R E = R(-0.066967f) * T + R(0.370275f);
-  return perez(A, B, C, D, E, ct, gamma, cg, ts, cts);
+  return perez(k.pl, d.z, m_acos(cg), cg);
 }
 
 /* sun_and_sky.glsl:229-245: sky radiance (linear RGB) in direction d */
-ASUNA_SKY_FN V<R> envColor(V<R> sun, V<R> d, R T) {
-  const R ts = m_acos(sun.z);
-  const R chi = (R(4.0f) / R(9.0f) - T / R(120.0f)) * (kPi<R>() - R(2) * ts);
-  R lum = R(1000.0f) * ((R(4.0453f) * T - R(4.9710f)) * m_tan(chi) - R(0.2155f) * T + R(2.4192f));
-  lum = lum * skyLuminance(d, sun, T);
-  const V<R> X = skyXYZ(d, sun, T, lum);
+ASUNA_SKY_FN V<R> envColor(const SkyConst<R>& k, V<R> d) {
+  const R lum = k.lum * skyLuminance(k, d);
+  const V<R> X = skyXYZ(k, d, lum);
   const V<R> c = v3(R(3.241f) * X.x - R(1.537f) * X.y - R(0.499f) * X.z,
                     R(-0.969f) * X.x + R(1.876f) * X.y + R(0.042f) * X.z,
                     R(0.056f) * X.x - R(0.204f) * X.y + R(1.057f) * X.z);
@@ -259,9 +283,10 @@ ASUNA_SKY_FN V<R> envColor(V<R> sun, V<R> d, R T) {
 ASUNA_SKY_FN V<R> irradiance(V<R> sun, R haze) {
   V<R> acc = v3(R(0), R(0), R(0));
   const V<R> n = v3(R(0), R(0), R(1.0f));
+  const SkyConst<R> k = skyConst(sun, haze);
   for (float u = 1.0f / 10.0f; u < 1.0f; u += 1.0f / 5.0f)
     for (float v = 1.0f / 10.0f; v < 1.0f; v += 1.0f / 5.0f)
-      acc = vadd(acc, envColor(sun, diffuseDir(n, R(u), R(v)), haze));
+      acc = vadd(acc, envColor(k, diffuseDir(n, R(u), R(v))));
   return v3(acc.x / R(25.0f), acc.y / R(25.0f), acc.z / R(25.0f));
 }
 
@@ -339,66 +364,98 @@ ASUNA_SKY_FN R nightAdjust(V<R> sd) {
   return f;
 }
 
-/* sun_and_sky.glsl:405-533: radiance of the sun & sky in direction d */
-ASUNA_SKY_FN V<R> sunAndSky(const Params<R>& ss, V<R> inDir) {
-  R factor = R(1.0f), nightFactor = R(1.0f);
+/* sun_and_sky.glsl:405-533, the part that does not depend on the direction:
+ * a renderer evaluates it once per scene (the ground's irradiance alone is 25
+ * evaluations of the sky). */
+template <class R>
+struct SkyState {
+  V<R> rgbScale, realSun, irr, ground, night;
+  V<R> sunUp, sunDown;  // sun colour for directions above the horizon, below it
+  SkyConst<R> k;
+  R hh, haze, sat, redblueshift, factor, blur;
+  R radius, glow, disk, sunZ;  // the sun's angular radius with its glow, glow and disk intensities, height
+  R glowScale, diskScale;      // of a physically scaled sun
+  int y_is_up, dark, has_disk;
+};
+ASUNA_SKY_FN SkyState<R> skyState(const Params<R>& ss) {
+  SkyState<R> s;
+  s.factor = R(1.0f);
   V<R> rgbScale = v3(ss.rgb[0], ss.rgb[1], ss.rgb[2]);
-  const R hh = ss.horizon_height / R(10.0f);
-  V<R> dir = vectorTweak(inDir, ss.y_is_up, hh);
+  s.hh = ss.horizon_height / R(10.0f);
+  s.y_is_up = ss.y_is_up;
   R haze = R(2.0f) + ss.haze;
   if (haze < R(2.0f)) haze = R(2.0f);
-  const R sat = tweakSaturation(ss.saturation, haze);
+  s.haze = haze;
+  s.sat = tweakSaturation(ss.saturation, haze);
+  s.redblueshift = ss.redblueshift;
   if (luminance(rgbScale) < R(0.0f)) {
-    const R s = R(1.0f) / R(80000.0f);
-    rgbScale = v3(s, s, s);
+    const R k = R(1.0f) / R(80000.0f);
+    rgbScale = v3(k, k, k);
   }
-  rgbScale = vscale(rgbScale, ss.multiplier);
-  if (ss.multiplier <= R(0.0f)) return v3(R(0), R(0), R(0));
+  s.rgbScale = vscale(rgbScale, ss.multiplier);
+  s.dark = ss.multiplier <= R(0.0f) ? 1 : 0;
+  V<R> sun = vnormalize(v3(ss.sun_dir[0], ss.sun_dir[1], ss.sun_dir[2]));
+  sun = vectorTweak(sun, ss.y_is_up, s.hh);
+  s.realSun = sun;
+  if (sun.z < R(0.001f)) {
+    if (sun.z < R(0.0f)) s.factor = nightAdjust(sun);
+    sun.z = R(0.001f);
+    sun = vnormalize(sun);
+  }
+  s.sunZ = sun.z;
+  s.k = skyConst(sun, haze);
+  s.sunUp = sunColor(sun, haze);
+  s.sunDown = sunColor(sun, R(2.0f));
+  s.has_disk = (ss.sun_disk_intensity > R(0.0f) && ss.sun_disk_scale > R(0.0f)) ? 1 : 0;
+  s.radius = R(0.00465f) * ss.sun_disk_scale * R(10.0f);
+  s.diskScale = s.glowScale = R(1.0f);
+  if (ss.physically_scaled_sun == 1)
+    physicalScale(ss.sun_disk_scale, ss.sun_glow_intensity, ss.sun_disk_intensity, s.diskScale, s.glowScale);
+  s.glow = ss.sun_glow_intensity;
+  s.disk = ss.sun_disk_intensity;
+  s.irr = irradiance(sun, R(2.0f));
+  s.ground = v3(ss.ground[0], ss.ground[1], ss.ground[2]);
+  s.night = v3(ss.night[0], ss.night[1], ss.night[2]);
+  s.blur = ss.horizon_blur / R(10.0f);
+  return s;
+}
+
+/* sun_and_sky.glsl:405-533: radiance of the sun & sky in direction d */
+ASUNA_SKY_FN V<R> sunAndSky(const SkyState<R>& s, V<R> inDir) {
+  R nightFactor = R(1.0f);
+  V<R> dir = vectorTweak(inDir, s.y_is_up, s.hh);
+  if (s.dark) return v3(R(0), R(0), R(0));
   const R downness = dir.z;
   const V<R> realDir = dir;
   if (dir.z < R(0.001f)) {
     dir.z = R(0.001f);
     dir = vnormalize(dir);
   }
-  V<R> sun = vnormalize(v3(ss.sun_dir[0], ss.sun_dir[1], ss.sun_dir[2]));
-  sun = vectorTweak(sun, ss.y_is_up, hh);
-  const V<R> realSun = sun;
-  if (sun.z < R(0.001f)) {
-    if (sun.z < R(0.0f)) factor = nightAdjust(sun);
-    sun.z = R(0.001f);
-    sun = vnormalize(sun);
-  }
   V<R> tint;
-  if (factor > R(0.0f)) {
-    tint = envColor(sun, dir, haze);
-    if (factor < R(1.0f)) tint = vscale(tint, factor);
+  if (s.factor > R(0.0f)) {
+    tint = envColor(s.k, dir);
+    if (s.factor < R(1.0f)) tint = vscale(tint, s.factor);
   } else {
     tint = v3(R(0), R(0), R(0));
   }
-  const V<R> sunCol = sunColor(sun, downness > R(0) ? haze : R(2.0f));
-  if (ss.sun_disk_intensity > R(0.0f) && ss.sun_disk_scale > R(0.0f)) {
-    const R angle = m_acos(vdot(realDir, realSun));
-    const R radius = R(0.00465f) * ss.sun_disk_scale * R(10.0f);
-    if (angle < radius) {
-      R diskScale = R(1.0f), glowScale = R(1.0f);
-      if (ss.physically_scaled_sun == 1)
-        physicalScale(ss.sun_disk_scale, ss.sun_glow_intensity, ss.sun_disk_intensity, diskScale, glowScale);
-      R f = (R(1.0f) - angle / radius) * R(10.0f);
-      f = (m_pow(f / R(10.0f), R(3.0f)) * R(2.0f) * ss.sun_glow_intensity * glowScale +
-           smoothstep_(R(8.5f), R(9.5f) + (haze / R(50.0f)), f) * R(100.0f) * ss.sun_disk_intensity * diskScale);
+  const V<R> sunCol = downness > R(0) ? s.sunUp : s.sunDown;
+  if (s.has_disk) {
+    const R angle = m_acos(vdot(realDir, s.realSun));
+    if (angle < s.radius) {
+      R f = (R(1.0f) - angle / s.radius) * R(10.0f);
+      f = (m_pow(f / R(10.0f), R(3.0f)) * R(2.0f) * s.glow * s.glowScale +
+           smoothstep_(R(8.5f), R(9.5f) + (s.haze / R(50.0f)), f) * R(100.0f) * s.disk * s.diskScale);
       tint = vadd(tint, vscale(sunCol, f));
     }
   }
-  V<R> out = vmul(tint, rgbScale);
+  V<R> out = vmul(tint, s.rgbScale);
   if (downness <= R(0.0f)) {
-    const V<R> irr = irradiance(sun, R(2.0f));
-    V<R> down = v3(ss.ground[0], ss.ground[1], ss.ground[2]);
-    down = vmul(down, vmul(vadd(irr, vscale(sunCol, sun.z)), rgbScale));
-    if (factor < R(1)) down = vscale(down, factor);
-    const R blur = ss.horizon_blur / R(10.0f);
-    if (blur > R(0.0f)) {
+    V<R> down = s.ground;
+    down = vmul(down, vmul(vadd(s.irr, vscale(sunCol, s.sunZ)), s.rgbScale));
+    if (s.factor < R(1)) down = vscale(down, s.factor);
+    if (s.blur > R(0.0f)) {
       R dn = -downness;
-      dn = dn / blur;
+      dn = dn / s.blur;
       if (dn > R(1.0f)) dn = R(1.0f);
       dn = smoothstep_(R(0.0f), R(1.0f), dn);
       out = vadd(vscale(out, R(1.0f) - dn), vscale(down, dn));
@@ -408,16 +465,17 @@ ASUNA_SKY_FN V<R> sunAndSky(const Params<R>& ss, V<R> inDir) {
       nightFactor = R(0.0f);
     }
   }
-  out = colorTweak(out, sat, ss.redblueshift);
+  out = colorTweak(out, s.sat, s.redblueshift);
   V<R> res = out;
   if (nightFactor > R(0.0f)) {
-    const V<R> night = vscale(v3(ss.night[0], ss.night[1], ss.night[2]), nightFactor);
+    const V<R> night = vscale(s.night, nightFactor);
     if (res.x < night.x) res.x = night.x;
     if (res.y < night.y) res.y = night.y;
     if (res.z < night.z) res.z = night.z;
   }
   return vscale(res, kPi<R>());
 }
+ASUNA_SKY_FN V<R> sunAndSky(const Params<R>& ss, V<R> inDir) { return sunAndSky(skyState(ss), inDir); }
 
 #undef ASUNA_SKY_FN
 
