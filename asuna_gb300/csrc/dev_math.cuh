@@ -250,7 +250,7 @@ __device__ __forceinline__ f3 uniformSampleSphere(f2 u) {
   return f3{r * mcos(phi), r * msin(phi), z};
 }
 // sun_and_sky.glsl:405-533 (include/asuna_sunsky.h) in world direction L
-__device__ __noinline__ f3 evalSunSky(const SceneDev& S, f3 L) {
+static __device__ __noinline__ f3 evalSunSky(const SceneDev& S, f3 L) {
   const asuna_sky::V<float> r = asuna_sky::sunAndSky<float>(S.skyState, asuna_sky::V<float>{L.x, L.y, L.z});
   return f3{r.x, r.y, r.z};
 }

@@ -193,6 +193,8 @@ enum CounterSlot {
   kCntFetchExtend = 3,
   kCntFetchShadow = 4,
   kCntCls0 = 5,  // rays per shading class (kNumShadeClasses slots)
+  kCntPass = 22,    // the current pass (see passOf)
+  kCntTicket = 23,  // blocks of the path kernel that are done
   kCntNum32 = 24
 };
 

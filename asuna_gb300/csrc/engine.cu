@@ -173,7 +173,9 @@ int asuna_ctx_create(int device_ordinal, asuna_ctx** out) {
   cudaDeviceProp prop;
   ASUNA_CUDA_TRY(cudaGetDeviceProperties(&prop, device_ordinal));
   c->numSMs = prop.multiProcessorCount;
-  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->bodyStream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return fail(ASUNA_ERR_CUDA, "cudaStreamCreate failed");
   }
@@ -185,6 +187,7 @@ int asuna_ctx_create(int device_ordinal, asuna_ctx** out) {
     cudaFreeHost(c->hostCnt);
     cudaFreeHost(c->hostErr);
     if (c->errEvent) cudaEventDestroy(c->errEvent);
+    cudaStreamDestroy(c->bodyStream);
     cudaStreamDestroy(c->stream);
     delete c;
     return fail(ASUNA_ERR_OOM, "counter allocation failed");
@@ -194,6 +197,7 @@ int asuna_ctx_create(int device_ordinal, asuna_ctx** out) {
   c->traceGrid = c->traceGridShadow = c->numSMs * traceBlocksPerSm();
   c->shadeGrid = c->numSMs * shadeBlocksPerSm();
   c->raygenGrid = c->numSMs * 16;
+  c->pathGrid = c->numSMs * pathBlocksPerSm();
   *out = c;
   return ASUNA_OK;
 }
@@ -211,6 +215,7 @@ int asuna_ctx_destroy(asuna_ctx* c) {
   if (c->hostCnt) cudaFreeHost(c->hostCnt);
   if (c->hostErr) cudaFreeHost(c->hostErr);
   if (c->errEvent) cudaEventDestroy(c->errEvent);
+  cudaStreamDestroy(c->bodyStream);
   cudaStreamDestroy(c->stream);
   delete c;
   return ASUNA_OK;
@@ -905,7 +910,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
   if (stats) ASUNA_CUDA_TRY(cudaMemsetAsync(c->cnt, 0, offsetof(DevCounters, stackOverflow), c->stream));
   // timing events: [begin, end] + one pair per extend / shade / connect launch
   size_t evNeed = 2;
-  for (auto& b : batches) evNeed += size_t(wavefrontPasses(b.maxDepth, s->view)) * 8;
+  for (auto& b : batches) evNeed += size_t(wavefrontPasses(b.maxDepth, s->view)) * 10;
   if (stats) {
     while (c->events.size() < evNeed) {
       cudaEvent_t ev;
@@ -916,6 +921,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
   }
   size_t evi = 2;
   std::vector<std::pair<int, size_t>> timed;  // (kind, first event index)
+  uint64_t launches = 0;                      // kernels of the recorded sequence
   // CUDA graph of the whole launch sequence, reused while the key matches
   const bool useGraph = c->graphs && !hostRecords;
   GraphEntry* hitEntry = nullptr;
@@ -925,7 +931,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     std::memcpy(key.data(), &s->view, sizeof(SceneDev));  // every scene pointer and size
     key.insert(key.end(), {uint64_t(uintptr_t(c->wave.base)), c->wave.capacity,
            uint64_t(uintptr_t(dShots)), uint64_t(uintptr_t(dRanges)), uint64_t(c->traceGrid), uint64_t(c->shadeGrid),
-           uint64_t(c->raygenGrid), uint64_t(c->counters), uint64_t(stats ? 1 : 0), uint64_t(c->refill[0]),
+           uint64_t(c->raygenGrid), uint64_t(c->pathGrid), uint64_t(c->counters), uint64_t(stats ? 1 : 0), uint64_t(c->refill[0]),
            uint64_t(c->refill[1]), uint64_t(c->speculate[0]), uint64_t(c->speculate[1]), uint64_t(c->occupancy),
            uint64_t(c->raySort), uint64_t(c->stackLimit), uint64_t(c->traceThreads), uint64_t(c->sharedStack),
            uint64_t(c->occupancyShadow), uint64_t(c->traceGridShadow)});
@@ -938,9 +944,12 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     hitEntry->lastUse = ++c->useClock;
     ASUNA_CUDA_TRY(cudaGraphLaunch(hitEntry->exec, c->stream));
     timed = hitEntry->timed;
+    launches = hitEntry->launches;
   } else {
   if (useGraph) ASUNA_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   bool evFail = false;
+  cudaError_t graphErr = cudaSuccess;
+  const bool loopGraph = useGraph && !stats && !c->counters && !c->raySort;
   KParams P{};
   P.S = s->view;
   P.W = c->wave.view;
@@ -957,47 +966,112 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     int rg = int(std::min<uint64_t>((b.paths + 255) / 256, uint64_t(c->raygenGrid)));
     launchRaygen(P, std::max(rg, 1), c->stream);
     const int passes = wavefrontPasses(b.maxDepth, s->view);
-    for (int depth = 1; depth <= passes; ++depth) {
-      P.depth = uint32_t(depth);
-      // inside a capture the events become event-record nodes of the graph,
-      // so every replay records them again
-      auto record = [&](cudaEvent_t ev) {
-        return useGraph ? cudaEventRecordWithFlags(ev, c->stream, cudaEventRecordExternal)
-                        : cudaEventRecord(ev, c->stream);
-      };
-      auto timedLaunch = [&](int kind, auto&& fn) {
-        if (stats && record(c->events[evi]) != cudaSuccess) evFail = true;
-        fn();
-        if (stats) {
-          if (record(c->events[evi + 1]) != cudaSuccess) evFail = true;
-          timed.push_back({kind, evi});
-          evi += 2;
-        }
-      };
-      if (c->raySort && depth >= 2) {
-        // sorted into the idle queue, which this pass then runs on
-        timedLaunch(3, [&] { launchSortQueue(P, c->raySort, c->raygenGrid, c->stream); });
-        P.cur ^= 1;
+    // inside a capture the events become event-record nodes of the graph,
+    // so every replay records them again
+    auto record = [&](cudaEvent_t ev) {
+      return useGraph ? cudaEventRecordWithFlags(ev, c->stream, cudaEventRecordExternal)
+                      : cudaEventRecord(ev, c->stream);
+    };
+    auto timedLaunch = [&](int kind, auto&& fn) {
+      if (stats && record(c->events[evi]) != cudaSuccess) evFail = true;
+      fn();
+      if (stats) {
+        if (record(c->events[evi + 1]) != cudaSuccess) evFail = true;
+        timed.push_back({kind, evi});
+        evi += 2;
       }
+    };
+    auto issuePass = [&](cudaStream_t st) {
       P.occupancy = c->occupancy;
       P.blockThreads = c->traceThreads;
       P.sharedStack = c->sharedStack;
       P.refillLanes = c->refill[0];
       P.speculate = c->speculate[0];
-      timedLaunch(0, [&] { launchExtend(P, c->traceGrid, c->stream); });
-      timedLaunch(1, [&] { launchShade(P, c->shadeGrid, c->stream); });
+      timedLaunch(0, [&] { launchExtend(P, c->traceGrid, st); });
+      timedLaunch(1, [&] { launchShade(P, c->shadeGrid, st); });
       P.refillLanes = c->refill[1];
       P.speculate = c->speculate[1];
       P.occupancy = c->occupancyShadow;
-      timedLaunch(2, [&] { launchConnect(P, c->traceGridShadow, c->stream); });
+      timedLaunch(2, [&] { launchConnect(P, c->traceGridShadow, st); });
+      launches += 2 + uint64_t(shadeLaunches(s->view.classMask));
+    };
+    // The path kernel takes over as soon as a pass has few enough rays (the
+    // instrumented traversal counts wavefront passes only).
+    const uint32_t most = c->counters ? 0u : pathMost(s->view.classMask);
+    launches += 2;
+    P.depth = 1;
+    if (b.paths <= most) {
+      timedLaunch(0, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
+      ++launches;
+    } else if (loopGraph && passes > 1) {
+      // The later passes as a loop in the graph that ends when no ray is left
+      // or the path kernel has taken the rest: passes are not issued (nor
+      // recorded) that have nothing to do.
+      issuePass(c->stream);
+      cudaStreamCaptureStatus cs;
+      cudaGraph_t graph = nullptr, body = nullptr;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t ndeps = 0;
+      cudaGraphConditionalHandle handle = 0;
+      cudaGraphNodeParams np = {};
+      cudaGraphNode_t node = nullptr;
+      P.cur = -1;
+      auto capture = [&](cudaError_t e) {
+        if (graphErr == cudaSuccess) graphErr = e;
+        return graphErr == cudaSuccess;
+      };
+      if (capture(cudaStreamGetCaptureInfo(c->stream, &cs, nullptr, &graph, nullptr, nullptr, nullptr)) &&
+          capture(cudaGraphConditionalHandleCreate(&handle, graph, 0, 0))) {
+        launchPath(P, passes, most, c->pathGrid, handle, c->stream);
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = handle;
+        np.conditional.type = cudaGraphCondTypeWhile;
+        np.conditional.size = 1;
+        if (capture(cudaStreamGetCaptureInfo(c->stream, &cs, nullptr, &graph, &deps, nullptr, &ndeps)) &&
+            capture(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &np)) &&
+            capture(cudaStreamUpdateCaptureDependencies(c->stream, &node, nullptr, 1,
+                                                        cudaStreamSetCaptureDependencies)) &&
+            capture(cudaStreamBeginCaptureToGraph(c->bodyStream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                  cudaStreamCaptureModeThreadLocal))) {
+          issuePass(c->bodyStream);
+          launchPath(P, passes, most, c->pathGrid, handle, c->bodyStream);
+          capture(cudaStreamEndCapture(c->bodyStream, &body));
+        }
+      }
+      launches += 2;
+      P.cur = 0;
+    } else {
+      issuePass(c->stream);
       P.cur ^= 1;
+      for (int depth = 2; depth <= passes; ++depth) {
+        P.depth = uint32_t(depth);
+        if (most) {
+          timedLaunch(0, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
+          ++launches;
+        }
+        if (c->raySort) {
+          // sorted into the idle queue, which this pass then runs on
+          timedLaunch(3, [&] { launchSortQueue(P, c->raySort, c->raygenGrid, c->stream); });
+          P.cur ^= 1;
+          launches += 3;
+        }
+        issuePass(c->stream);
+        P.cur ^= 1;
+      }
     }
     launchAccumulate(P, b.maxPix, P.W.numRanges, c->stream);
-    if (hostRecords) launchRecords(P, dRec + b.pathOffset, c->raygenGrid, c->stream);
+    if (hostRecords) {
+      launchRecords(P, dRec + b.pathOffset, c->raygenGrid, c->stream);
+      ++launches;
+    }
   }
   if (useGraph) {
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
+    if (e == cudaSuccess && graphErr != cudaSuccess) {
+      cudaGraphDestroy(graph);
+      e = graphErr;
+    }
     if (e != cudaSuccess) return fail(ASUNA_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
     if (evFail) {
       cudaGraphDestroy(graph);
@@ -1009,6 +1083,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     if (e != cudaSuccess) return fail(ASUNA_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(e));
     g.key = key;
     g.timed = timed;
+    g.launches = launches;
     g.lastUse = ++c->useClock;
     if (c->gcache.size() >= 8) {
       auto lru = std::min_element(c->gcache.begin(), c->gcache.end(),
@@ -1046,11 +1121,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     stats->tris_tested = c->hostCnt->tris;
     stats->shadow_nodes_visited = c->hostCnt->shNodes;
     stats->shadow_tris_tested = c->hostCnt->shTris;
-    // raygen + accumulate (+ records) per wave; extend, shading, connect per depth
-    for (const Batch& b : batches)
-      stats->kernel_launches += 2 + (hostRecords ? 1 : 0) +
-                                uint64_t(wavefrontPasses(b.maxDepth, s->view)) * (2 + shadeLaunches(s->view.classMask)) +
-                                (c->raySort ? 3 * uint64_t(wavefrontPasses(b.maxDepth, s->view) - 1) : 0);
+    stats->kernel_launches = launches;
     float ms = 0;
     ASUNA_CUDA_TRY(cudaEventElapsedTime(&ms, c->events[0], c->events[1]));
     stats->ms_total = ms;

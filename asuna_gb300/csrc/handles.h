@@ -19,15 +19,18 @@ struct GraphEntry {
   std::vector<uint64_t> key;
   cudaGraphExec_t exec = nullptr;
   std::vector<std::pair<int, size_t>> timed;  // (kernel kind, first event index)
+  uint64_t launches = 0;
   uint64_t lastUse = 0;
 };
 
 struct asuna_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t bodyStream = nullptr;  // captures the graphs' repeated passes; nothing runs on it
   int numSMs = 0;
   int traceGrid = 0, shadeGrid = 0, raygenGrid = 0;
   int traceGridShadow = 0;  // the occlusion pass's traversal grid
+  int pathGrid = 0;         // the path kernel's
   int traceBlocksCap = 0;   // asuna_ctx_set_launch's traversal blocks per SM (0 = all that fit)
   asuna::DevCounters* cnt = nullptr;
   asuna::DevCounters* hostCnt = nullptr;
@@ -48,7 +51,15 @@ struct asuna_ctx {
   int32_t occupancyShadow = 8;  // the same for the occlusion pass
   int32_t traceThreads = 128;  // traversal kernel variant: threads per block
   int32_t sharedStack = 24;    // traversal kernel variant: stack entries in shared memory
-  int32_t raySort = 3;    // extend-queue sort mode before secondary passes (0 off)
+  // extend-queue sort mode before secondary passes (0 off).  Off by default:
+  // with the 8-wide nodes the sort gains the extend pass 5% at most and costs
+  // as much (21M-triangle scene, ms per render sorted / unsorted: 8 frames
+  // 19.2 / 18.8, 256 frames 434.7 / 434.0; a 320x180 preview 1.29 / 1.13).
+  // extend-queue sort mode before secondary passes (0 off).  Off by default:
+  // with the 8-wide nodes the sort gains the extend pass 5% at most and costs
+  // as much (21M-triangle scene, ms per render sorted / unsorted: 8 frames
+  // 21.9 / 21.7, 256 frames 434.7 / 434.0; a 1280x720 frame 2.23 / 2.05).
+  int32_t raySort = 0;
   int32_t stackLimit = 0; // traversal stack entries a ray may use (0 = the compiled capacity)
   int32_t bvhBuild = 0;   // bottom-level BVHs: 0 built on the device, 1 on host threads
   // traversals cut short on the device: the cumulative device count is

@@ -10,7 +10,7 @@ struct KParams {
   SceneDev S;
   WaveDev W;
   uint32_t depth;  // bounce being processed (1-based)
-  int32_t cur;     // extend queue holding this bounce's rays (0/1)
+  int32_t cur;     // extend queue holding this bounce's rays (0/1); -1: both from the counters (passOf)
   int32_t records; // write per-path parity records
   int32_t counters;
   uint32_t refillLanes;  // traversal: idle lanes of a warp that trigger a queue fetch
@@ -20,6 +20,19 @@ struct KParams {
   int32_t blockThreads;  // traversal: threads per block (64, 128, 256; 0 = 128)
   int32_t sharedStack;   // traversal: stack entries in shared memory (16, 24, 32; 0 = 24)
 };
+
+// The wavefront pass that a kernel works on.  A pass that a graph repeats
+// while rays are left finds its number in the counters; without the queue
+// sort the queues alternate with it.
+struct Pass {
+  uint32_t wave;
+  int cur;
+};
+__device__ __forceinline__ Pass passOf(const KParams& P) {
+  if (P.cur >= 0) return Pass{P.depth, P.cur};
+  const uint32_t w = P.W.cnt->c[kCntPass];
+  return Pass{w, int((w - 1u) & 1u)};
+}
 
 constexpr int kTraceThreads = 128;
 constexpr int kTraceMinBlocks = 8;   // resident blocks per SM the traversal kernels are compiled for
@@ -41,6 +54,15 @@ void launchAccumulate(const KParams& P, uint32_t maxPix, uint32_t nranges, cudaS
 void launchSortQueue(const KParams& P, int mode, int grid, cudaStream_t s);
 void launchRecords(const KParams& P, asuna_path_record* out, int grid, cudaStream_t s);
 void launchExtend(const KParams& P, int grid, cudaStream_t s);
+// The path kernel: follows the rays of pass P.depth (queue P.cur) to pass
+// `lastPass` if there are at most `most`, and empties the queue.  With a
+// conditional `handle` it works on the pass after the counters' one, makes
+// that the current pass and sets the condition to whether it has rays left.
+void launchPath(const KParams& P, int lastPass, uint32_t most, int grid, cudaGraphConditionalHandle handle,
+                cudaStream_t s);
+// rays up to which the path kernel is faster than wavefront passes
+uint32_t pathMost(uint32_t classMask);
+int pathBlocksPerSm();
 void launchConnect(const KParams& P, int grid, cudaStream_t s);
 // resident blocks per SM of the traversal variant (occupancy class 8/10/12 =
 // 32/40/48 resident warps, block size, shared-memory stack entries)

@@ -182,7 +182,9 @@ int renderNoAlloc(const asuna_scene* s, const asuna_shot* shot, asuna_film* film
   k_noallocBegin<<<1, 32, 0, stream>>>(dShot, sd, W.cnt);
 
   // batches of whole frames, each with its range record written in order
-  const int traceGrid = numSMs * traceBlocksPerSm(), shadeGrid = numSMs * 8, raygenGrid = numSMs * 16;
+  const int traceGrid = numSMs * traceBlocksPerSm(), shadeGrid = numSMs * 8, raygenGrid = numSMs * 16,
+            pathGrid = numSMs * pathBlocksPerSm();
+  const uint32_t most = pathMost(s->view.classMask);
   const int maxDepth = shot->state.max_path_depth;
   W.ranges = dRanges;
   W.numRanges = 1;
@@ -200,8 +202,12 @@ int renderNoAlloc(const asuna_scene* s, const asuna_shot* shot, asuna_film* film
     P.depth = 0;
     const int rg = int(std::min<uint64_t>((W.numPaths + 255) / 256, uint64_t(raygenGrid)));
     launchRaygen(P, std::max(rg, 1), stream);
-    for (int depth = 1; depth <= wavefrontPasses(maxDepth, s->view); ++depth) {
+    const int passes = wavefrontPasses(maxDepth, s->view);
+    for (int depth = 1; depth <= passes; ++depth) {
       P.depth = uint32_t(depth);
+      // (the path kernel takes the rest of the wave once it is small enough)
+      if (depth > 1 || W.numPaths <= most) launchPath(P, passes, most, pathGrid, 0, stream);
+      if (W.numPaths <= most) break;
       launchExtend(P, traceGrid, stream);
       launchShade(P, shadeGrid, stream);
       launchConnect(P, traceGrid, stream);
