@@ -144,6 +144,18 @@ int reportTraversal(asuna_ctx* c) {
               c->stackLimit > 0 ? c->stackLimit : kStackDepth, d);
 }
 
+void destroyStreams(asuna_ctx* c) {
+  for (ShadeFork& f : c->fork) {
+    for (int k = 0; k < kShadeForks; ++k) {
+      if (f.stream[k]) cudaStreamDestroy(f.stream[k]);
+      if (f.end[k]) cudaEventDestroy(f.end[k]);
+    }
+    if (f.begin) cudaEventDestroy(f.begin);
+  }
+  if (c->bodyStream) cudaStreamDestroy(c->bodyStream);
+  if (c->stream) cudaStreamDestroy(c->stream);
+}
+
 struct Batch {
   uint32_t rangeBegin, rangeEnd;
   uint32_t paths;
@@ -173,9 +185,16 @@ int asuna_ctx_create(int device_ordinal, asuna_ctx** out) {
   cudaDeviceProp prop;
   ASUNA_CUDA_TRY(cudaGetDeviceProperties(&prop, device_ordinal));
   c->numSMs = prop.multiProcessorCount;
-  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&c->bodyStream, cudaStreamNonBlocking) != cudaSuccess) {
-    if (c->stream) cudaStreamDestroy(c->stream);
+  bool made = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&c->bodyStream, cudaStreamNonBlocking) == cudaSuccess;
+  for (ShadeFork& f : c->fork) {
+    made = made && cudaEventCreateWithFlags(&f.begin, cudaEventDisableTiming) == cudaSuccess;
+    for (int k = 0; k < kShadeForks; ++k)
+      made = made && cudaStreamCreateWithFlags(&f.stream[k], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&f.end[k], cudaEventDisableTiming) == cudaSuccess;
+  }
+  if (!made) {
+    destroyStreams(c);
     delete c;
     return fail(ASUNA_ERR_CUDA, "cudaStreamCreate failed");
   }
@@ -187,8 +206,7 @@ int asuna_ctx_create(int device_ordinal, asuna_ctx** out) {
     cudaFreeHost(c->hostCnt);
     cudaFreeHost(c->hostErr);
     if (c->errEvent) cudaEventDestroy(c->errEvent);
-    cudaStreamDestroy(c->bodyStream);
-    cudaStreamDestroy(c->stream);
+    destroyStreams(c);
     delete c;
     return fail(ASUNA_ERR_OOM, "counter allocation failed");
   }
@@ -215,8 +233,7 @@ int asuna_ctx_destroy(asuna_ctx* c) {
   if (c->hostCnt) cudaFreeHost(c->hostCnt);
   if (c->hostErr) cudaFreeHost(c->hostErr);
   if (c->errEvent) cudaEventDestroy(c->errEvent);
-  cudaStreamDestroy(c->bodyStream);
-  cudaStreamDestroy(c->stream);
+  destroyStreams(c);
   delete c;
   return ASUNA_OK;
 }
@@ -988,7 +1005,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
       P.refillLanes = c->refill[0];
       P.speculate = c->speculate[0];
       timedLaunch(0, [&] { launchExtend(P, c->traceGrid, st); });
-      timedLaunch(1, [&] { launchShade(P, c->shadeGrid, st); });
+      timedLaunch(1, [&] { launchShade(P, c->shadeGrid, st, &c->fork[st == c->bodyStream ? 1 : 0]); });
       P.refillLanes = c->refill[1];
       P.speculate = c->speculate[1];
       P.occupancy = c->occupancyShadow;

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "dev_types.h"
+#include "kernels.h"
 
 struct WaveAlloc {
   void* base = nullptr;
@@ -27,6 +28,9 @@ struct asuna_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t bodyStream = nullptr;  // captures the graphs' repeated passes; nothing runs on it
+  // side streams of the shading classes: a stream belongs to one capture at a
+  // time, so the graphs' repeated passes have their own
+  asuna::ShadeFork fork[2];
   int numSMs = 0;
   int traceGrid = 0, shadeGrid = 0, raygenGrid = 0;
   int traceGridShadow = 0;  // the occlusion pass's traversal grid

@@ -45,7 +45,15 @@ constexpr int kShadeMinBlocks = 3;   // resident 256-thread blocks per SM the sh
 // rounding; waits for the stream)
 int prepareSky(SceneDev& S, cudaStream_t s);
 void launchRaygen(const KParams& P, int grid, cudaStream_t s);
-void launchShade(const KParams& P, int grid, cudaStream_t s);
+// Streams and events for the shading classes of a pass to run side by side:
+// one for every class but the pass's own stream's (a scene of twelve classes,
+// 480x270, 4 frames: 4.22 ms in a row, 3.30 on 3 side streams, 3.03 on 11).
+constexpr int kShadeForks = kNumShadeClasses - 1;
+struct ShadeFork {
+  cudaStream_t stream[kShadeForks] = {};
+  cudaEvent_t begin = nullptr, end[kShadeForks] = {};
+};
+void launchShade(const KParams& P, int grid, cudaStream_t s, const ShadeFork* fork = nullptr);
 // kernels launchShade issues for a scene's class mask (classify included)
 int shadeLaunches(uint32_t classMask);
 void launchAccumulate(const KParams& P, uint32_t maxPix, uint32_t nranges, cudaStream_t s);

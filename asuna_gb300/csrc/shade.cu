@@ -280,22 +280,39 @@ int prepareSky(SceneDev& S, cudaStream_t s) {
 
 void launchRaygen(const KParams& P, int grid, cudaStream_t s) { k_raygen<<<grid, 256, 0, s>>>(P); }
 // classify, then one kernel per shading class the scene's materials can
-// reach (each a persistent grid over its own list)
-void launchShade(const KParams& P, int grid, cudaStream_t s) {
+// reach (each a persistent grid over its own list).  The classes are
+// independent of each other: with `fork` they run side by side from three
+// classes on (two gain nothing), so that a pass with few rays waits for the
+// slowest class instead of for their sum.
+void launchShade(const KParams& P, int grid, cudaStream_t s, const ShadeFork* fork) {
   k_classify<<<grid, 256, 0, s>>>(P);
   const uint32_t m = P.S.classMask | (1u << kClsTerminal);
-  if (m & (1u << kClsTerminal)) k_shadeClass<kClsTerminal><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsLambertian)) k_shadeClass<kClsLambertian><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsRoughPlastic)) k_shadeClass<kClsRoughPlastic><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsDielectric)) k_shadeClass<kClsDielectric><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsPlastic)) k_shadeClass<kClsPlastic><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsMirror)) k_shadeClass<kClsMirror><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsConductor)) k_shadeClass<kClsConductor><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsRoughConductor)) k_shadeClass<kClsRoughConductor><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsPhong)) k_shadeClass<kClsPhong><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsPbr)) k_shadeClass<kClsPbr><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsDisney)) k_shadeClass<kClsDisney><<<grid, 256, 0, s>>>(P);
-  if (m & (1u << kClsKang18)) k_shadeClass<kClsKang18><<<grid, 256, 0, s>>>(P);
+  const int nc = __builtin_popcount(m), lanes = fork && nc > 2 ? (nc < kShadeForks + 1 ? nc : kShadeForks + 1) : 1;
+  if (lanes > 1) {
+    cudaEventRecord(fork->begin, s);
+    for (int k = 0; k + 1 < lanes; ++k) cudaStreamWaitEvent(fork->stream[k], fork->begin, 0);
+  }
+  int at = 0;
+  auto next = [&] {
+    const int k = at++ % lanes;
+    return k == 0 ? s : fork->stream[k - 1];
+  };
+  if (m & (1u << kClsTerminal)) k_shadeClass<kClsTerminal><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsLambertian)) k_shadeClass<kClsLambertian><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsRoughPlastic)) k_shadeClass<kClsRoughPlastic><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsDielectric)) k_shadeClass<kClsDielectric><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsPlastic)) k_shadeClass<kClsPlastic><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsMirror)) k_shadeClass<kClsMirror><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsConductor)) k_shadeClass<kClsConductor><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsRoughConductor)) k_shadeClass<kClsRoughConductor><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsPhong)) k_shadeClass<kClsPhong><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsPbr)) k_shadeClass<kClsPbr><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsDisney)) k_shadeClass<kClsDisney><<<grid, 256, 0, next()>>>(P);
+  if (m & (1u << kClsKang18)) k_shadeClass<kClsKang18><<<grid, 256, 0, next()>>>(P);
+  for (int k = 0; k + 1 < lanes; ++k) {
+    cudaEventRecord(fork->end[k], fork->stream[k]);
+    cudaStreamWaitEvent(s, fork->end[k], 0);
+  }
 }
 int shadeLaunches(uint32_t classMask) { return 1 + __builtin_popcount(classMask | (1u << kClsTerminal)); }
 int shadeBlocksPerSm() {

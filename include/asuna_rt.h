@@ -387,7 +387,7 @@ int asuna_ctx_set_traversal_occupancy(asuna_ctx* ctx, int extend_blocks_per_sm, 
 /* Reorders the extend queue before every secondary pass by direction and
  * origin so warps carry rays that walk alike: 0 off, 1 octant x 4 x 4 x 4
  * origin cells, 2 octant x 8 x 8 x 8 cells in Morton order, 3 the same with
- * the origin cell major (the default).  Results do not depend on it. */
+ * the origin cell major.  Off by default.  Results do not depend on it. */
 int asuna_ctx_set_ray_sort(asuna_ctx* ctx, int mode);
 /* Caps the traversal stack at `entries` per ray (1..64; 0 = 64, the
  * compiled capacity, which every scene asuna_scene_create accepts fits).
