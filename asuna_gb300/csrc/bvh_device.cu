@@ -384,7 +384,18 @@ __global__ void k_primBounds(const VtxDev* __restrict__ vtx, const uint4* __rest
     cen[p] = make_float4(c[0], c[1], c[2], 0.0f);
     ord0[p] = p;
   }
-  // per-mesh bounds: one atomic per warp when the whole warp is in one mesh
+  // per-mesh bounds: at most one atomic per warp when the whole warp is in
+  // one mesh, and none where the bound as last seen already covers it (bounds
+  // only grow, so a stale value costs an atomic at worst; 21M triangles:
+  // 4.8 -> 3.6 ms)
+  auto extend = [](uint32_t* dst, int k, uint32_t v) {
+    const uint32_t seen = __ldcg(&dst[k]);
+    if (isMinWord(k)) {
+      if (v < seen) atomicMin(&dst[k], v);
+    } else if (v > seen) {
+      atomicMax(&dst[k], v);
+    }
+  };
   const unsigned lane = threadIdx.x & 31u;
   const int m0 = __shfl_sync(0xffffffffu, m, 0);
   const bool uniform = __all_sync(0xffffffffu, !valid || m == m0);
@@ -403,15 +414,11 @@ __global__ void k_primBounds(const VtxDev* __restrict__ vtx, const uint4* __rest
       }
     if (lane == 0 && valid) {
       uint32_t* dst = meshKeys + size_t(m0) * 12;
-      for (int k = 0; k < 12; ++k) {
-        if (isMinWord(k)) atomicMin(&dst[k], key[k]); else atomicMax(&dst[k], key[k]);
-      }
+      for (int k = 0; k < 12; ++k) extend(dst, k, key[k]);
     }
   } else if (valid) {
     uint32_t* dst = meshKeys + size_t(m) * 12;
-    for (int k = 0; k < 12; ++k) {
-      if (isMinWord(k)) atomicMin(&dst[k], key[k]); else atomicMax(&dst[k], key[k]);
-    }
+    for (int k = 0; k < 12; ++k) extend(dst, k, key[k]);
   }
 }
 

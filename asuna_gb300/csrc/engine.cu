@@ -674,18 +674,10 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
       off += n;
     }
   }
-  std::vector<float4> env(1, make_float4(0, 0, 0, 0));
-  std::vector<float2> marg(1, make_float2(0, 0)), cond(1, make_float2(0, 0));
-  if (d->envmap.rgba && d->envmap.width && d->envmap.height) {
+  const bool hasEnv = d->envmap.rgba && d->envmap.width && d->envmap.height;
+  if (hasEnv) {
     ew = d->envmap.width;
     eh = d->envmap.height;
-    const size_t np = size_t(ew) * eh;
-    env.resize(np);
-    std::memcpy(env.data(), d->envmap.rgba, np * 16);
-    marg.resize(np);
-    cond.resize(np);
-    asuna_envmap_tables(ew, eh, d->envmap.rgba, reinterpret_cast<float*>(marg.data()),
-                        reinterpret_cast<float*>(cond.data()));
   }
   // ---- binary trees of both levels -> wide nodes ----
   if (onDevice) {
@@ -719,11 +711,38 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
   if ((rc = devUpload(s, inst.data(), inst.size(), &v.inst)) ||
       (rc = devUpload(s, mats.data(), mats.size(), &v.mats)) ||
       (rc = devUpload(s, lights.data(), lights.size(), &v.lights)) ||
-      (rc = devUpload(s, env.data(), env.size(), &v.env)) || (rc = devUpload(s, marg.data(), marg.size(), &v.marg)) ||
-      (rc = devUpload(s, cond.data(), cond.size(), &v.cond)) ||
       (rc = devUpload(s, texels.data(), texels.size(), &v.texels)) ||
       (rc = devUpload(s, texInfo.data(), texInfo.size(), &v.texInfo)))
     return rc;
+  {
+    // Importance tables on the device from this many texels on: the host
+    // takes 34 ns a texel (4.5 ms for 512x256), the launches and the temporary
+    // memory about 0.1 ms.
+    constexpr size_t kDeviceEnv = 4096;
+    const size_t np = size_t(ew) * eh;
+    const float4 black = make_float4(0, 0, 0, 0);
+    std::vector<float2> marg, cond;
+    const bool tables = hasEnv && np >= kDeviceEnv;
+    if (!tables) {
+      marg.resize(np);
+      cond.resize(np);
+      if (hasEnv)
+        asuna_envmap_tables(ew, eh, d->envmap.rgba, reinterpret_cast<float*>(marg.data()),
+                            reinterpret_cast<float*>(cond.data()));
+    }
+    const float4* texels4 = hasEnv ? reinterpret_cast<const float4*>(d->envmap.rgba) : &black;
+    if ((rc = devUpload(s, tables ? nullptr : texels4, np, &v.env)) ||
+        (rc = devUpload(s, tables ? nullptr : marg.data(), np, &v.marg)) ||
+        (rc = devUpload(s, tables ? nullptr : cond.data(), np, &v.cond)))
+      return rc;
+    if (tables) {
+      ASUNA_CUDA_TRY(cudaMemcpyAsync(const_cast<float4*>(v.env), texels4, np * sizeof(float4), cudaMemcpyHostToDevice,
+                                     c->stream));
+      if ((rc = prepareEnvTables(v.env, int(ew), int(eh), const_cast<float2*>(v.marg), const_cast<float2*>(v.cond),
+                                 c->stream)))
+        return rc;
+    }
+  }
   v.tlasRoot = int32_t(wideRoots.size() - 1);
   std::memset(&v.sky, 0, sizeof(v.sky));
   if (d->sun_and_sky && d->sun_and_sky->in_use == 1) {

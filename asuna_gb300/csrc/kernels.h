@@ -44,6 +44,8 @@ constexpr int kShadeMinBlocks = 3;   // resident 256-thread blocks per SM the sh
 // S.skyState of S.sky (evaluated on the device, with the shading kernels'
 // rounding; waits for the stream)
 int prepareSky(SceneDev& S, cudaStream_t s);
+// the importance tables of an uploaded W x H environment map (waits for the stream)
+int prepareEnvTables(const float4* env, int W, int H, float2* marg, float2* cond, cudaStream_t s);
 void launchRaygen(const KParams& P, int grid, cudaStream_t s);
 // Streams and events for the shading classes of a pass to run side by side:
 // one for every class but the pass's own stream's (a scene of twelve classes,
