@@ -11,8 +11,9 @@
 // stage, so weights are fetched once per 128 T pixels.  The input channels
 // are consumed in groups of 16 (K = 16 per MMA):
 //   * activations: for each 8-channel chunk, one TMA tiled load of the
-//     18 x (8T + 2) halo of the tiles from the NHWC tensor (zero fill outside
-//     the image) lands as [row][col][8] bf16 (slots padded to 128 B); for tap
+//     18 x (8T + 2) halo of the tiles (zero fill outside the image), from
+//     rows [P][C] or, as the denoiser keeps its activations, from planes
+//     [C / 8][P][8], lands as [row][col][8] bf16 (slots padded to 128 B); for tap
 //     (dy, dx) and tile t the A operand is the view starting at pixel
 //     (dy, dx + 8t) of that halo: 8-row core matrices are 8 consecutive
 //     pixels of one image row, image rows are (8T + 2) * 16 B apart (stride
@@ -27,10 +28,18 @@
 // The CTAs are persistent and warp-specialised: one elected thread of a
 // fifth warp issues the copies and one of a sixth the MMAs of a stream of
 // units (the ring runs ahead across unit boundaries, the MMAs alternate
-// between two TMEM accumulator buffers); the four epilogue warps read their 32 TMEM lanes
-// each (tcgen05.ld) of the finished buffer, apply bias, ReLU and the ReLU
+// between two TMEM accumulator buffers); the four epilogue warps read their 32
+// TMEM lanes each (tcgen05.ld) of the finished buffer, apply bias, ReLU and the ReLU
 // mask, store bf16 (or fp32) and hand the buffer back, while the next unit's
-// MMAs run.  Every mbarrier wait is bounded: on expiry the CTA records an
+// MMAs run.  What the network does between two convolutions goes with the
+// first one's epilogue: the 2x2 mean, the 2x upsampling into the decoder's
+// input, the final exponential (a 1080p image: 10 launches and 230 us of
+// copies, pooling and output kernels; the convolutions themselves take 757 ->
+// 652 us with those in them, as planes load and store whole lines).
+//
+// Four CTAs per SM (80 registers a thread) are what hides one tile's epilogue
+// behind the others' copies and MMAs: at 118 registers, two CTAs, the image
+// took 930 us instead of 752.  Every mbarrier wait is bounded: on expiry the CTA records an
 // error, stops its work and still frees its tensor memory.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -41,10 +50,12 @@
 #include <cstdlib>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 
 #include "../../include/asuna_denoise.h"
 #include "common.h"
+#include "conv_tc.h"
 
 namespace asuna {
 namespace tc {
@@ -54,7 +65,10 @@ constexpr int kTileH = 16, kTileW = 8;                         // pixels per MMA
 constexpr int kHaloH = kTileH + 2;
 constexpr int kMaxTiles = 4;                                   // tiles per CTA, side by side in x
 constexpr int kMaxStages = 8;  // copy-ring depth, chosen per layer in [2, 8]
-constexpr int kHeader = 256;   // barriers, the TMEM address and the abort flag
+constexpr int kBarriers = 256;  // barriers, the TMEM address and the abort flag
+constexpr int kEpiWarps = 4;
+// then each epilogue warp's copy of the slice's bias
+__host__ __device__ constexpr int headerBytes(int nt) { return kBarriers + kEpiWarps * nt * 4; }
 // One TMA box of 8 channels covers the halo of T tiles: 18 x (8T + 2) pixels
 // of 16 bytes; its shared-memory slot is padded to 128 bytes.
 __host__ __device__ constexpr int haloW(int T) { return kTileW * T + 2; }
@@ -74,7 +88,7 @@ __host__ __device__ constexpr int wStage(int nt) { return 9 * 2 * nt * 16; }  //
 // S ring stages of activations; weights either in the ring (a stage per
 // group) or resident (all `groups` of the layer, loaded once per CTA)
 size_t smemFor(int nt, int T, int S, bool resident, int groups) {
-  return kHeader + size_t(S) * actStage(T) + size_t(resident ? groups : S) * wStage(nt);
+  return headerBytes(nt) + size_t(S) * actStage(T) + size_t(resident ? groups : S) * wStage(nt);
 }
 uint32_t pow2Cols(int n) {
   uint32_t c = 32;
@@ -188,6 +202,20 @@ __device__ __forceinline__ void mma(uint32_t tmem, uint64_t a, uint64_t b, uint3
 __device__ __forceinline__ uint64_t descPlus(uint64_t d, uint32_t units) {
   return (d & 0xFFFFFFFF00000000ull) | uint64_t(uint32_t(d) + units);
 }
+// v twice, to 32 aligned bytes
+__device__ __forceinline__ void storePair(uint4* p, uint4 v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
+               "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void exchange(uint32_t& x, uint32_t& y, bool on) {
+  const uint32_t t = on ? y : x;
+  y = on ? x : y;
+  x = t;
+}
+__device__ __forceinline__ float2 unpack2(uint32_t u) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+}
 __device__ __forceinline__ void commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -209,14 +237,22 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float* v) {
 struct TcArgs {
   const __nv_bfloat16* wt;    // [cout/nt][cin/16][9][2][nt][8]
   const float* bias;          // [cout] or null
-  const __nv_bfloat16* mask;  // [P][cout] or null
-  void* out;                  // [P][cout]
+  const uint4* mask;          // laid out as out, or null
+  void* out;                  // or null
+  uint4* pool;                // [cout / 8][P / 4] or null
+  uint4* up;                  // [cout / 8][4 P] or null
+  float4* head;               // [P] or null
+  float4* image;              // [n][imgH][imgW] or null
+  const float4* radiance;
+  int imgH, imgW;
   int n, h, w, cin, cout;
   int nt, slices;             // output channels per CTA, cout / nt
   int tiles;                  // 16 x 8 pixel tiles per unit, side by side in x (the kernel's T)
   int tilesX, tilesY;         // units (16 x 8 tiles pixels) per image row / column
   int units;                  // tilesX * tilesY * n * slices
   int relu, outF32;
+  int planes;                 // in, mask and out are [c / 8][P][8] (else [P][c])
+  size_t chunkStride, pixStride;  // of mask and bf16 out, in 16-byte chunks
   uint32_t tmemCols;          // two accumulator buffers of tiles * nt columns
   uint32_t wStageBytes;       // 9 * 2 * nt * 16
   int stages;                 // copy-ring depth
@@ -272,7 +308,6 @@ __device__ __forceinline__ void mbarArrive(uint32_t bar) {
 // MMAs.  Barriers: full / empty per ring stage (copies landed / MMAs done
 // reading), accFull / accEmpty per accumulator buffer, drain (every MMA of
 // the CTA done, before TMEM is freed).
-constexpr int kEpiWarps = 4;
 constexpr int kProducerWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
 constexpr int kThreads = 32 * (kEpiWarps + 2);
 
@@ -285,7 +320,7 @@ constexpr int kThreads = 32 * (kEpiWarps + 2);
 // channels each, so that more SMs share a layer) measured 16.2 us for the same
 // tile: a group's weights then are 18 copies, which one thread issues.
 template <int T>
-__global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__ CUtensorMap act, TcArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__ CUtensorMap act, TcArgs a) {
   extern __shared__ __align__(1024) unsigned char sm[];
   // [0, 128): barriers, the TMEM address and the abort flag; then the
   // activation stages and the weight stages
@@ -297,11 +332,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__
   uint64_t* wFull = drain + 1;  // resident weights landed
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(wFull + 1);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
-  static_assert((2 * kMaxStages + 6) * 8 + 8 <= kHeader, "barrier header");
+  static_assert((2 * kMaxStages + 6) * 8 + 8 <= kBarriers, "barrier header");
   constexpr int hw = haloW(T);
   constexpr uint32_t chunk = uint32_t(chunkBytes(T)), stageA = uint32_t(actStage(T));
   const int S = a.stages;
-  unsigned char* actBase = sm + kHeader;
+  unsigned char* actBase = sm + headerBytes(a.nt);
   unsigned char* wBase = actBase + S * stageA;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -357,8 +392,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__
         const uint32_t bar = smem(&full[s]);
         mbarExpectTx(bar, uint32_t(2 * boxBytes(T)) + (a.resident ? 0u : a.wStageBytes));
         const uint32_t dstA = smem(actBase + s * stageA);
-        tmaLoad4d(dstA, &act, g * 16, U.x0 - 1, U.y0 - 1, U.img, bar);
-        tmaLoad4d(dstA + chunk, &act, g * 16 + 8, U.x0 - 1, U.y0 - 1, U.img, bar);
+        if (a.planes) {  // (four 32-bit words per pixel: x stays 16-byte aligned)
+          tmaLoad4d(dstA, &act, 4 * (U.x0 - 1), U.y0 - 1, U.img, 2 * g, bar);
+          tmaLoad4d(dstA + chunk, &act, 4 * (U.x0 - 1), U.y0 - 1, U.img, 2 * g + 1, bar);
+        } else {
+          tmaLoad4d(dstA, &act, g * 16, U.x0 - 1, U.y0 - 1, U.img, bar);
+          tmaLoad4d(dstA + chunk, &act, g * 16 + 8, U.x0 - 1, U.y0 - 1, U.img, bar);
+        }
         if (!a.resident)
           bulkLoad(smem(wBase + size_t(s) * a.wStageBytes),
                    a.wt + (size_t(U.slice) * size_t(groups) + size_t(g)) * (a.wStageBytes / 2), a.wStageBytes, bar);
@@ -436,6 +476,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__
   } else {
     // epilogue: warp w owns TMEM lanes 32w..32w+31 = pixels 32w..32w+31 of each tile
     const int m = warp * 32 + lane;
+    // this warp's copy of the bias: with the whole L1 given to the ring, global
+    // loads per 16 channels came from L2 each time (a layer of 128 channels at
+    // 12x16 pixels: 15.1 -> 13.0 us)
+    float* sBias = reinterpret_cast<float*>(sm + kBarriers) + warp * a.nt;
+    int slice = -1;
     for (int k = 0; k < myUnits; ++k) {
       const uint32_t buf = uint32_t(k & 1);
       if (!mbarWaitOr(smem(&accFull[buf]), uint32_t(k >> 1) & 1u, abortFlag)) {
@@ -445,22 +490,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__
       fenceAfter();
       const Unit U = unitOf(a, int(blockIdx.x) + k * int(gridDim.x));
       const int n0 = U.slice * a.nt;
+      if (a.bias && U.slice != slice) {
+        slice = U.slice;
+        __syncwarp();
+        for (int i = lane; i < a.nt; i += 32) sBias[i] = a.bias[n0 + i];
+        __syncwarp();
+      }
       const uint32_t laneBase = tmem + (uint32_t(warp * 32) << 16) + buf * bufCols;
       for (int t2 = 0; t2 < T; ++t2)
         for (int c0 = 0; c0 < a.nt; c0 += 16) {
           const int py = U.y0 + m / kTileW, px = U.x0 + kTileW * t2 + m % kTileW;
           const bool inside = py < a.h && px < a.w;
-          // 16 consecutive channels of one pixel: 32 B (bf16) or 64 B (f32),
-          // aligned as cout and n0 + c0 are multiples of 16
-          const size_t e = ((size_t(U.img) * a.h + py) * a.w + px) * size_t(a.cout) + size_t(n0 + c0);
+          const size_t pix = (size_t(U.img) * a.h + py) * a.w + px;
+          // 16 channels of one pixel: two 16-byte chunks, aligned as n0 + c0
+          // is a multiple of 16; in planes the lanes' chunks are consecutive
+          const size_t e = size_t((n0 + c0) / 8) * a.chunkStride + pix * a.pixStride;
           float v[16];
+          __syncwarp();
           ld16(laneBase + uint32_t(t2 * a.nt + c0), v);
-          if (!inside) continue;
           if (a.bias) {
-            const float4* b4 = reinterpret_cast<const float4*>(a.bias + n0 + c0);
+            const float4* b4 = reinterpret_cast<const float4*>(sBias + c0);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float4 b = __ldg(&b4[i]);
+              const float4 b = b4[i];
               v[4 * i] += b.x;
               v[4 * i + 1] += b.y;
               v[4 * i + 2] += b.z;
@@ -471,26 +523,89 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_tc(const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
           }
-          if (a.mask) {
-            const uint4* m4 = reinterpret_cast<const uint4*>(a.mask + e);
-            const uint4 mm[2] = {m4[0], m4[1]};
+          if (a.mask && inside) {
+            const uint4 mm[2] = {a.mask[e], a.mask[e + a.chunkStride]};
             const __nv_bfloat16* mk = reinterpret_cast<const __nv_bfloat16*>(mm);
 #pragma unroll
             for (int i = 0; i < 16; ++i)
               if (!(__bfloat162float(mk[i]) > 0.0f)) v[i] = 0.0f;
           }
           if (a.outF32) {
-            float4* o4 = reinterpret_cast<float4*>(static_cast<float*>(a.out) + e);
+            if (inside) {
+              float4* o4 = reinterpret_cast<float4*>(static_cast<float*>(a.out) + pix * size_t(a.cout) + n0 + c0);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o4[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          } else {
-            uint4 pk[2];
-            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(pk);
+              for (int i = 0; i < 4; ++i) o4[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+            continue;
+          }
+          if (a.head) {
+            if (inside && n0 + c0 == 0) a.head[pix] = make_float4(v[0], v[1], v[2], 0.0f);
+            continue;
+          }
+          if (a.image) {
+            if (py < a.imgH && px < a.imgW && n0 + c0 == 0) {
+              const size_t q = (size_t(U.img) * a.imgH + py) * a.imgW + px;
+              const float4 r = a.radiance[q];  // (may be the image itself)
+              a.image[q] = make_float4(fmaxf(expm1f(v[0] + log1pf(fmaxf(r.x, 0.0f))), 0.0f),
+                                       fmaxf(expm1f(v[1] + log1pf(fmaxf(r.y, 0.0f))), 0.0f),
+                                       fmaxf(expm1f(v[2] + log1pf(fmaxf(r.z, 0.0f))), 0.0f), 1.0f);
+            }
+            continue;
+          }
+          uint4 pk[2];
+          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(pk);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) h2[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            uint4* o4 = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + e);
+          for (int i = 0; i < 8; ++i) h2[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+          if (a.out && inside) {
+            uint4* o4 = static_cast<uint4*>(a.out) + e;
             o4[0] = pk[0];
-            o4[1] = pk[1];
+            o4[a.chunkStride] = pk[1];
+          }
+          if (a.up && inside) {
+            // a row's two copies are 32 aligned bytes, one store (112 -> 48
+            // channels at 544x960, upsampled: 59 -> 45 us against two)
+            const size_t P4 = 4 * a.chunkStride;
+            uint4* o4 = a.up + size_t((n0 + c0) / 8) * P4 + (size_t(U.img) * a.h + py) * a.w * 4 + 2 * px;
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int y = 0; y < 2; ++y) storePair(o4 + c * P4 + size_t(y) * 2 * a.w, pk[c]);
+          }
+          if (a.pool) {
+            // A window's four pixels are lanes id = 0..3 (x first) of a group
+            // 1 and 8 lanes apart.  Each lane averages a quarter of the
+            // channels, words [2 id, 2 id + 2): it permutes its words to
+            // w[2 (k ^ id)], sends the pair that belongs to lane id ^ k in
+            // exchange k, and orders what it has by pixel again.  (Every lane
+            // fetching all words of three others took 24 shuffles, not 6: 80
+            // -> 67 us for 32 -> 32 channels at 1088x1920.)
+            uint32_t q[8];
+            memcpy(q, pk, sizeof(q));
+            const bool idX = lane & 1, idY = lane & kTileW;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              exchange(q[i], q[2 + i], idX);
+              exchange(q[4 + i], q[6 + i], idX);
+              exchange(q[i], q[4 + i], idY);
+              exchange(q[2 + i], q[6 + i], idY);
+              q[2 + i] = __shfl_xor_sync(0xffffffffu, q[2 + i], 1);
+              q[4 + i] = __shfl_xor_sync(0xffffffffu, q[4 + i], kTileW);
+              q[6 + i] = __shfl_xor_sync(0xffffffffu, q[6 + i], kTileW + 1);
+              exchange(q[i], q[2 + i], idX);
+              exchange(q[4 + i], q[6 + i], idX);
+              exchange(q[i], q[4 + i], idY);
+              exchange(q[2 + i], q[6 + i], idY);
+              const float2 p0 = unpack2(q[i]), p1 = unpack2(q[2 + i]), p2 = unpack2(q[4 + i]), p3 = unpack2(q[6 + i]);
+              const __nv_bfloat162 r = __floats2bfloat162_rn(
+                  __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(p0.x, p1.x), p2.x), p3.x)),
+                  __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(p0.y, p1.y), p2.y), p3.y)));
+              q[i] = *reinterpret_cast<const uint32_t*>(&r);
+            }
+            if (inside) {  // (h and w are even: a window is inside or outside)
+              const size_t chunk4 = size_t((n0 + c0) / 8 + (idY ? 1 : 0)) * (a.chunkStride / 4) +
+                                    ((size_t(U.img) * (a.h / 2) + py / 2) * (a.w / 2) + px / 2);
+              reinterpret_cast<uint2*>(a.pool)[2 * chunk4 + (idX ? 1 : 0)] = make_uint2(q[0], q[1]);
+            }
           }
         }
       // this warp's lanes of the buffer are read: hand it back to the MMAs
@@ -539,30 +654,21 @@ EncodeTiledFn encodeFn() {
 }  // namespace tc
 }  // namespace asuna
 
-using namespace asuna;
-using namespace asuna::tc;
+namespace asuna {
+namespace tc {
 
-extern "C" {
-
-int asuna_nn_weights_tc(void* stream, const void* w, void* wtc, int cout, int cin) {
-  if (!w || !wtc || cin % 16 || cout % 16) return fail(ASUNA_ERR_INVALID, "asuna_nn_weights_tc: bad argument");
-  const int n = cout * 9 * cin;
-  k_weights_tc<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wtc), cout, cin, sliceWidth(cout));
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? ASUNA_OK : fail(ASUNA_ERR_CUDA, "asuna_nn_weights_tc: %s", cudaGetErrorString(e));
-}
-
-int asuna_nn_conv3x3_tc(void* stream, const void* in, int n, int h, int w, int cin, const void* weight_tc,
-                        const float* bias, int cout, int relu, const void* mask, void* out, int out_f32) {
-  if (!in || !weight_tc || !out || n <= 0 || h <= 0 || w <= 0)
-    return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: bad argument");
+int conv3x3(cudaStream_t s, const Conv& c) {
+  const int n = c.n, h = c.h, w = c.w, cin = c.cin, cout = c.cout;
   if (cin % 16 || cout % 16)
     return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: cin %% 16 and cout %% 16 required");
   // the copies and the epilogue's 16-byte loads and stores need 16-byte bases
-  if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weight_tc) | reinterpret_cast<uintptr_t>(bias) |
-       reinterpret_cast<uintptr_t>(mask) | reinterpret_cast<uintptr_t>(out)) % 16)
-    return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: operands must be 16-byte aligned");
+  uintptr_t bits = 0;
+  for (const void* p : {c.in, c.weights, static_cast<const void*>(c.bias), c.mask, static_cast<const void*>(c.out),
+                        static_cast<const void*>(c.pool), static_cast<const void*>(c.up),
+                        static_cast<const void*>(c.head), static_cast<const void*>(c.image),
+                        static_cast<const void*>(c.radiance)})
+    bits |= reinterpret_cast<uintptr_t>(p);
+  if (bits % 16) return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: operands must be 16-byte aligned");
   EncodeTiledFn enc = encodeFn();
   if (!enc) return fail(ASUNA_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
   int dev = 0, sms = 1, smemSm = 0, reserve = 0;
@@ -581,21 +687,36 @@ int asuna_nn_conv3x3_tc(void* stream, const void* in, int n, int h, int w, int c
                       int(std::min<long long>(4, (units + sms - 1) / sms)));
   }
   const int T = shape.T;
-  // NHWC bf16 as a 4-D tensor (C, W, H, N); box = 8 channels x the T tiles' halo
+  // Rows: the 4-D tensor (C, W, H, N) of bf16, box = 8 channels x the T tiles'
+  // halo.  Planes: (4 W, H, N, C / 8) of 32-bit words, whose box has whole
+  // rows of the halo as its innermost extent: one request of 16 (8 T + 2)
+  // bytes where rows take 8 T + 2 requests of 16 bytes.
   CUtensorMap map;
-  const cuuint64_t dims[4] = {cuuint64_t(cin), cuuint64_t(w), cuuint64_t(h), cuuint64_t(n)};
-  const cuuint64_t strides[3] = {cuuint64_t(cin) * 2, cuuint64_t(w) * cin * 2, cuuint64_t(h) * w * cin * 2};
-  const cuuint32_t box[4] = {8, cuuint32_t(haloW(T)), kHaloH, 1};
+  const cuuint64_t W = cuuint64_t(w), H = cuuint64_t(h), N = cuuint64_t(n), C = cuuint64_t(cin);
+  const cuuint64_t dimsR[4] = {C, W, H, N}, dimsP[4] = {4 * W, H, N, C / 8};
+  const cuuint64_t stridesR[3] = {C * 2, W * C * 2, H * W * C * 2}, stridesP[3] = {16 * W, 16 * W * H, 16 * W * H * N};
+  const cuuint32_t boxR[4] = {8, cuuint32_t(haloW(T)), kHaloH, 1}, boxP[4] = {4 * cuuint32_t(haloW(T)), kHaloH, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(in), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = enc(&map, c.planes ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+                         const_cast<void*>(c.in), c.planes ? dimsP : dimsR, c.planes ? stridesP : stridesR,
+                         c.planes ? boxP : boxR, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: tensor map encoding failed (%d)", int(r));
   TcArgs a{};
-  a.wt = static_cast<const __nv_bfloat16*>(weight_tc);
-  a.bias = bias;
-  a.mask = static_cast<const __nv_bfloat16*>(mask);
-  a.out = out;
+  a.wt = static_cast<const __nv_bfloat16*>(c.weights);
+  a.bias = c.bias;
+  a.mask = static_cast<const uint4*>(c.mask);
+  a.out = c.out;
+  a.pool = static_cast<uint4*>(c.pool);
+  a.up = static_cast<uint4*>(c.up);
+  a.head = c.head;
+  a.image = c.image;
+  a.radiance = c.radiance;
+  a.imgH = c.imgH;
+  a.imgW = c.imgW;
+  a.planes = c.planes ? 1 : 0;
+  a.chunkStride = c.planes ? size_t(n) * h * w : 1;
+  a.pixStride = c.planes ? 1 : size_t(cout) / 8;
   a.n = n;
   a.h = h;
   a.w = w;
@@ -604,8 +725,8 @@ int asuna_nn_conv3x3_tc(void* stream, const void* in, int n, int h, int w, int c
   a.tiles = T;
   a.tilesX = (w + kTileW * T - 1) / (kTileW * T);
   a.tilesY = (h + kTileH - 1) / kTileH;
-  a.relu = relu;
-  a.outF32 = out_f32;
+  a.relu = c.relu ? 1 : 0;
+  a.outF32 = c.f32 ? 1 : 0;
   a.nt = nt;
   a.slices = cout / a.nt;
   a.tmemCols = pow2Cols(2 * T * nt);
@@ -630,10 +751,46 @@ int asuna_nn_conv3x3_tc(void* stream, const void* in, int n, int h, int w, int c
   // when there is less work
   const int perSm = shape.perSm;
   const long long grid = std::min<long long>(units, (long long)sms * perSm);
-  kernels[size_t(T - 1)]<<<unsigned(std::max<long long>(grid, 1)), kThreads, smemBytes,
-                           static_cast<cudaStream_t>(stream)>>>(map, a);
+  kernels[size_t(T - 1)]<<<unsigned(std::max<long long>(grid, 1)), kThreads, smemBytes, s>>>(map, a);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? ASUNA_OK : fail(ASUNA_ERR_CUDA, "asuna_nn_conv3x3_tc: %s", cudaGetErrorString(e));
+}
+
+}  // namespace tc
+}  // namespace asuna
+
+using namespace asuna;
+using namespace asuna::tc;
+
+extern "C" {
+
+int asuna_nn_weights_tc(void* stream, const void* w, void* wtc, int cout, int cin) {
+  if (!w || !wtc || cin % 16 || cout % 16) return fail(ASUNA_ERR_INVALID, "asuna_nn_weights_tc: bad argument");
+  const int n = cout * 9 * cin;
+  k_weights_tc<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wtc), cout, cin, sliceWidth(cout));
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ASUNA_OK : fail(ASUNA_ERR_CUDA, "asuna_nn_weights_tc: %s", cudaGetErrorString(e));
+}
+
+int asuna_nn_conv3x3_tc(void* stream, const void* in, int n, int h, int w, int cin, const void* weight_tc,
+                        const float* bias, int cout, int relu, const void* mask, void* out, int out_f32) {
+  if (!in || !weight_tc || !out || n <= 0 || h <= 0 || w <= 0)
+    return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_tc: bad argument");
+  Conv c;
+  c.in = in;
+  c.n = n;
+  c.h = h;
+  c.w = w;
+  c.cin = cin;
+  c.weights = weight_tc;
+  c.bias = bias;
+  c.cout = cout;
+  c.relu = relu != 0;
+  c.mask = mask;
+  c.out = out;
+  c.f32 = out_f32 != 0;
+  return conv3x3(static_cast<cudaStream_t>(stream), c);
 }
 
 int asuna_nn_tc_status(int* expired) {

@@ -2,15 +2,19 @@
 // inference): a U-Net over the radiance / albedo / normal images, standing in
 // for the reference's OptiX AOV denoiser (src/tracer/denoiser.cpp:143-224).
 //
-// Tensors are NHWC bf16 with channel counts padded to multiples of 16; all
-// products accumulate in fp32.  The 3x3 convolution is an implicit GEMM
-// (M = pixels, N = output channels, K = 9 taps x input channels) on
-// mma.sync.m16n8k16 bf16 tensor-core instructions, fed by a 3-stage cp.async
-// pipeline (zero-fill for the halo) and ldmatrix fragment loads; bias, ReLU
-// and the ReLU mask of the backward pass are fused into the epilogue.  The
-// input gradient is the same kernel on flipped, transposed weights; the
-// weight gradient is a split-K GEMM over pixels (ldmatrix.trans fragments,
-// fp32 atomics into the weight-gradient buffer).
+// The network's activations are bf16 in planes of eight channels ([C / 8][P][8],
+// P pixels; channel counts padded to multiples of 16): a convolution's loads
+// and stores then are whole lines, and an upsampled level and a skip connection
+// lie side by side without a copy.  The entry points on single operations take
+// rows (NHWC).  All products accumulate in fp32.  The 3x3 convolution is the
+// tcgen05 kernel of conv_tc.cu or an implicit GEMM (M = pixels, N = output
+// channels, K = 9 taps x input channels) on mma.sync.m16n8k16 bf16 tensor-core
+// instructions, fed by a 3-stage cp.async pipeline (zero-fill for the halo) and
+// ldmatrix fragment loads; bias, ReLU and the ReLU mask of the backward pass
+// are fused into the epilogue.  The input gradient is the same kernel on
+// flipped, transposed weights; the weight gradient is a split-K GEMM over
+// pixels (ldmatrix.trans fragments, fp32 atomics into the weight-gradient
+// buffer).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -24,6 +28,7 @@
 
 #include "../../include/asuna_denoise.h"
 #include "common.h"
+#include "conv_tc.h"
 #include "handles.h"
 
 namespace asuna {
@@ -63,14 +68,24 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, const uint
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// Where channel c of pixel p of an activation lies: in rows ([P][C]) or in
+// planes of eight channels ([C / 8][P][8], the network's own activations).
+struct Layout {
+  size_t pix, chunk;  // halves from pixel to pixel, from 8 channels to the next 8
+  __device__ __forceinline__ size_t at(size_t p, int c) const { return p * pix + size_t(c >> 3) * chunk + (c & 7); }
+};
+Layout rowsOf(int c) { return {size_t(c), 8}; }
+Layout planesOf(size_t P) { return {8, 8 * P}; }
+
 struct ConvArgs {
-  const __nv_bfloat16* in;  // [P][Cin]
+  const __nv_bfloat16* in;
   const __nv_bfloat16* w;   // [Cout][9][Cin]
   const float* bias;        // [Cout] or null
-  const __nv_bfloat16* mask;  // [P][Cout] or null: out *= (mask > 0)
-  void* out;                // [P][Cout] bf16, or fp32 when outF32
+  const __nv_bfloat16* mask;  // laid out as out, or null: out *= (mask > 0)
+  void* out;                // bf16, or fp32 [P][Cout] when outF32
   int N, H, W, Cin, Cout;
   int relu, outF32;
+  Layout inL, outL;
 };
 
 // Forward 3x3 convolution, stride 1, zero padding 1.
@@ -102,7 +117,7 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a) {
     const int ys = ay + dy, xs = ax + dx;
     const bool va = ap < P && ys >= 0 && ys < a.H && xs >= 0 && xs < a.W;
     const __nv_bfloat16* srcA =
-        va ? a.in + ((size_t(an) * a.H + ys) * a.W + xs) * a.Cin + c0 + ah : a.in;
+        va ? a.in + a.inL.at((size_t(an) * a.H + ys) * a.W + xs, c0 + ah) : a.in;
     cpAsync16(&sA[stage][ar * kLds + ah], srcA, va);
     if (tid < 2 * kBN) {
       const bool vb = bco < a.Cout;
@@ -170,7 +185,7 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a) {
           v1 = fmaxf(v1, 0.0f);
         }
         if (a.mask) {
-          const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(a.mask + size_t(p) * a.Cout + co);
+          const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(a.mask + a.outL.at(size_t(p), co));
           if (!(__bfloat162float(m.x) > 0.0f)) v0 = 0.0f;
           if (!(__bfloat162float(m.y) > 0.0f)) v1 = 0.0f;
         }
@@ -179,20 +194,27 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a) {
           *o = make_float2(v0, v1);
         } else {
           __nv_bfloat162* o =
-              reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(a.out) + size_t(p) * a.Cout + co);
+              reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(a.out) + a.outL.at(size_t(p), co));
           *o = __floats2bfloat162_rn(v0, v1);
         }
       }
     }
 }
 
+void launchConv(cudaStream_t s, const ConvArgs& a) {
+  const int P = a.N * a.H * a.W;
+  dim3 g((P + kBM - 1) / kBM, (a.Cout + kBN - 1) / kBN);
+  k_conv3x3<<<g, 256, 0, s>>>(a);
+}
+
 struct WgradArgs {
-  const __nv_bfloat16* dz;  // [P][Cout]
-  const __nv_bfloat16* x;   // [P][Cin]
+  const __nv_bfloat16* dz;
+  const __nv_bfloat16* x;
   float* dw;                // [Cout][9][Cin], accumulated
   float* db;                // [Cout], accumulated, or null
   int N, H, W, Cin, Cout;
   int pixelsPerBlock;
+  Layout dzL, xL;
 };
 
 constexpr int kWBK = 32;   // pixels per K step
@@ -219,12 +241,14 @@ __global__ void __launch_bounds__(256) k_conv3x3_wgrad(WgradArgs a) {
   const int steps = pBegin < pEnd ? (pEnd - pBegin + kWBK - 1) / kWBK : 0;
   const bool bias = a.db && blockIdx.y == 0 && tid < 64;
   // loads: 32 pixel rows x 64 channels = 256 x 16 B for each operand
-  const int lr = tid >> 3, lc = (tid & 7) * 8;
+  // (a warp takes 32 pixels of a plane, or 4 rows)
+  const bool planes = a.xL.pix == 8;
+  const int lr = planes ? lane : tid >> 3, lc = (planes ? warp : tid & 7) * 8;
   auto load = [&](int buf, int p0) {
     const int p = p0 + lr;
     // A: dz row
     const bool vaRow = p < pEnd && co0 + lc < a.Cout;
-    cpAsync16(&sA[buf][lr * kWLds + lc], vaRow ? a.dz + size_t(p) * a.Cout + co0 + lc : a.dz, vaRow);
+    cpAsync16(&sA[buf][lr * kWLds + lc], vaRow ? a.dz + a.dzL.at(size_t(p), co0 + lc) : a.dz, vaRow);
     // B: shifted x row
     bool vb = p < pEnd && ci0 + lc < a.Cin;
     const __nv_bfloat16* src = a.x;
@@ -232,7 +256,7 @@ __global__ void __launch_bounds__(256) k_conv3x3_wgrad(WgradArgs a) {
       const int n = p / (a.H * a.W), rem = p - n * a.H * a.W;
       const int y = rem / a.W + dy, xx = rem % a.W + dx;
       vb = y >= 0 && y < a.H && xx >= 0 && xx < a.W;
-      if (vb) src = a.x + ((size_t(n) * a.H + y) * a.W + xx) * a.Cin + ci0 + lc;
+      if (vb) src = a.x + a.xL.at((size_t(n) * a.H + y) * a.W + xx, ci0 + lc);
     }
     cpAsync16(&sB[buf][lr * kWLds + lc], src, vb);
   };
@@ -313,13 +337,13 @@ int wgradChunk(int P, int blocks) {
 }
 
 int launchWgrad(cudaStream_t s, const void* dz, const void* x, int n, int h, int w, int cin, int cout, float* dw,
-                float* db) {
+                float* db, bool planes) {
   const int P = n * h * w;
   dim3 g((cout + 63) / 64, 9 * ((cin + 63) / 64));
   const int chunk = wgradChunk(P, int(g.x * g.y));
   g.z = (P + chunk - 1) / chunk;
   WgradArgs a{static_cast<const __nv_bfloat16*>(dz), static_cast<const __nv_bfloat16*>(x), dw, db, n, h, w, cin, cout,
-              chunk};
+              chunk, planes ? planesOf(size_t(P)) : rowsOf(cout), planes ? planesOf(size_t(P)) : rowsOf(cin)};
   k_conv3x3_wgrad<<<g, 256, 0, s>>>(a);
   return int(cudaGetLastError());
 }
@@ -450,8 +474,18 @@ __global__ void k_avgpool2_v(const uint4* in, uint4* out, I N, I H, I W, I C8) {
   }
 }
 
+// r where the mask's channel is positive, else 0
+__device__ __forceinline__ void masked8(Bf8& r, uint4 mask) {
+  const Bf8 m = unpack8(mask);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (!(m.v[k] > 0.0f)) r.v[k] = 0.0f;
+}
+
+// `mask` (laid out as din, or null): a ReLU's output that din is the gradient of
 template <typename I>
-__global__ void k_avgpool2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, I C8, int accumulate) {
+__global__ void k_avgpool2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, I C8, int accumulate,
+                                 const uint4* mask) {
   const I total = N * H * W * C8;
   for (I i = I(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += I(gridDim.x) * blockDim.x) {
     const I c = i % C8, q = i / C8, x = q % W, t = q / W, y = t % H, n = t / H;
@@ -465,6 +499,7 @@ __global__ void k_avgpool2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, I
 #pragma unroll
       for (int k = 0; k < 8; ++k) r.v[k] = __fmul_rn(0.25f, g.v[k]);
     }
+    if (mask) masked8(r, __ldg(&mask[i]));
     din[i] = pack8(r);
   }
 }
@@ -479,7 +514,8 @@ __global__ void k_upsample2_v(const uint4* in, uint4* out, I N, I H, I W, I C8, 
 }
 
 template <typename I>
-__global__ void k_upsample2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, I C8, I Ct8, I cOff8) {
+__global__ void k_upsample2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, I C8, I Ct8, I cOff8,
+                                  const uint4* mask) {
   const I total = N * H * W * C8;  // H, W of the (small) input
   for (I i = I(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += I(gridDim.x) * blockDim.x) {
     const I c = i % C8, q = i / C8, x = q % W, t = q / W, y = t % H, n = t / H;
@@ -490,6 +526,7 @@ __global__ void k_upsample2_bwd_v(const uint4* dout, uint4* din, I N, I H, I W, 
     Bf8 r;
 #pragma unroll
     for (int k = 0; k < 8; ++k) r.v[k] = __fadd_rn(__fadd_rn(__fadd_rn(a0.v[k], a1.v[k]), a2.v[k]), a3.v[k]);
+    if (mask) masked8(r, __ldg(&mask[i]));
     din[i] = pack8(r);
   }
 }
@@ -514,32 +551,14 @@ __global__ void k_copy_channels_v(const uint4* src, I Cs8, I sOff8, uint4* dst, 
   }
 }
 
-// decoder input in one pass: out[p] = (up2(low)[p] channels 0..Cu, skip[p]
-// channels 0..Cs); every chunk of out written once, in order
-template <typename I>
-__global__ void k_upsample_concat_v(const uint4* low, const uint4* skip, uint4* out, I N, I H, I W, I Cu8, I Cs8) {
-  const I Ct8 = Cu8 + Cs8, total = N * H * W * Ct8;
-  for (I i = I(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += I(gridDim.x) * blockDim.x) {
-    const I c = i % Ct8, q = i / Ct8;
-    uint4 v;
-    if (c < Cu8) {
-      const I x = q % W, t = q / W, y = t % H, n = t / H;
-      v = __ldg(&low[((n * (H / 2) + y / 2) * (W / 2) + x / 2) * Cu8 + c]);
-    } else {
-      v = __ldg(&skip[q * Cs8 + (c - Cu8)]);
-    }
-    out[i] = v;
-  }
-}
-
 // Network input: log1p(radiance), albedo, normal, log2(1 + filter-weight
 // sum) / 16 (the sample count: how much noise there is to remove), the
 // per-pixel noise as log1p of the mean over rgb of the input radiance's
 // standard-deviation estimate, and a flag that the noise is known (1) or
-// not (0, no estimate given); zeros up to C; pixels outside the h x w image
-// (padding up to hp x wp) are zero.
+// not (0, no estimate given); zeros up to 16 channels, in two planes; pixels
+// outside the h x w image (padding up to hp x wp) are zero.
 __global__ void k_prep_input(const float4* rad, const float4* alb, const float4* nrm, const float4* wsum,
-                             const float4* noise, __nv_bfloat16* out, int n, int h, int w, int hp, int wp, int C) {
+                             const float4* noise, uint4* out, int n, int h, int w, int hp, int wp) {
   const size_t P = size_t(n) * hp * wp;
   for (size_t q = blockIdx.x * size_t(blockDim.x) + threadIdx.x; q < P; q += size_t(gridDim.x) * blockDim.x) {
     const int x = int(q % wp), y = int((q / wp) % hp), b = int(q / (size_t(wp) * hp));
@@ -569,9 +588,14 @@ __global__ void k_prep_input(const float4* rad, const float4* alb, const float4*
         v[11] = 1.0f;
       }
     }
-    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + q * C);
-    for (int c = 0; c < C; c += 2)
-      o[c / 2] = __floats2bfloat162_rn(c < 12 ? v[c] : 0.0f, c + 1 < 12 ? v[c + 1] : 0.0f);
+    Bf8 lo, hi;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      lo.v[k] = v[k];
+      hi.v[k] = k < 4 ? v[8 + k] : 0.0f;
+    }
+    out[q] = pack8(lo);
+    out[P + q] = pack8(hi);
   }
 }
 
@@ -591,7 +615,7 @@ __global__ void k_half_noise(const float4* a, const float4* b, float4* half, flo
 // L1 loss on log radiance with the residual connection:
 //   y_c = head_c + log1p(rad_c),  loss += |y_c - log1p(target_c)|  (c < 3)
 // and its gradient with respect to head (sign / count; zero elsewhere).
-__global__ void k_l1_loss(const float* head, int C, const float4* rad, const float4* target, __nv_bfloat16* grad,
+__global__ void k_l1_loss(const float* head, int C, const float4* rad, const float4* target, uint4* grad,
                           int n, int h, int w, int hp, int wp, float invCount, float* loss) {
   const size_t P = size_t(n) * hp * wp;
   float s = 0.0f;
@@ -608,10 +632,8 @@ __global__ void k_l1_loss(const float* head, int C, const float4* rad, const flo
         g[c] = d > 0.0f ? invCount : (d < 0.0f ? -invCount : 0.0f);
       }
     }
-    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(grad + q * C);
-    o[0] = __floats2bfloat162_rn(g[0], g[1]);
-    o[1] = __floats2bfloat162_rn(g[2], 0.0f);
-    for (int c = 4; c < C; c += 2) o[c / 2] = __floats2bfloat162_rn(0.0f, 0.0f);
+    grad[q] = pack8({{g[0], g[1], g[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}});
+    grad[P + q] = make_uint4(0u, 0u, 0u, 0u);
   }
   for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
@@ -624,7 +646,7 @@ __global__ void k_l1_loss(const float* head, int C, const float4* rad, const flo
 // loss converges to the median, which sits below the mean of right-skewed
 // radiance noise).  dL/dhead = 2 (o - t) (o + 1) / (o + 0.01)^2 where o > 0.
 __global__ void k_relmse_loss(const float* head, int C, const float4* rad, const float4* target,
-                              __nv_bfloat16* grad, int n, int h, int w, int hp, int wp, float invCount, float* loss) {
+                              uint4* grad, int n, int h, int w, int hp, int wp, float invCount, float* loss) {
   const size_t P = size_t(n) * hp * wp;
   float s = 0.0f;
   for (size_t q = blockIdx.x * size_t(blockDim.x) + threadIdx.x; q < P; q += size_t(gridDim.x) * blockDim.x) {
@@ -643,10 +665,8 @@ __global__ void k_relmse_loss(const float* head, int C, const float4* rad, const
         g[c] = e > 0.0f ? 2.0f * d * (e + 1.0f) * den * invCount : 0.0f;
       }
     }
-    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(grad + q * C);
-    o[0] = __floats2bfloat162_rn(g[0], g[1]);
-    o[1] = __floats2bfloat162_rn(g[2], 0.0f);
-    for (int c = 4; c < C; c += 2) o[c / 2] = __floats2bfloat162_rn(0.0f, 0.0f);
+    grad[q] = pack8({{g[0], g[1], g[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}});
+    grad[P + q] = make_uint4(0u, 0u, 0u, 0u);
   }
   for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
@@ -815,10 +835,8 @@ int asuna_nn_conv3x3(void* stream, const void* in, int n, int h, int w, int cin,
     return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3: bad argument");
   if (cin % 16 || cout % 8) return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3: cin %% 16 and cout %% 8 must be 0");
   ConvArgs a{static_cast<const __nv_bfloat16*>(in), static_cast<const __nv_bfloat16*>(weight), bias,
-             static_cast<const __nv_bfloat16*>(mask), out, n, h, w, cin, cout, relu, out_f32};
-  const int P = n * h * w;
-  dim3 g((P + kBM - 1) / kBM, (cout + kBN - 1) / kBN);
-  k_conv3x3<<<g, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+             static_cast<const __nv_bfloat16*>(mask), out, n, h, w, cin, cout, relu, out_f32, rowsOf(cin), rowsOf(cout)};
+  launchConv(static_cast<cudaStream_t>(stream), a);
   NN_CHECK_LAUNCH();
 }
 
@@ -826,7 +844,7 @@ int asuna_nn_conv3x3_wgrad(void* stream, const void* dz, const void* x, int n, i
                            float* dweight) {
   clearError();
   if (!dz || !x || !dweight || cin % 16 || cout % 8) return fail(ASUNA_ERR_INVALID, "asuna_nn_conv3x3_wgrad: bad argument");
-  if (launchWgrad(static_cast<cudaStream_t>(stream), dz, x, n, h, w, cin, cout, dweight, nullptr))
+  if (launchWgrad(static_cast<cudaStream_t>(stream), dz, x, n, h, w, cin, cout, dweight, nullptr, false))
     return fail(ASUNA_ERR_CUDA, "asuna_nn_conv3x3_wgrad: launch failed");
   return ASUNA_OK;
 }
@@ -861,7 +879,7 @@ int asuna_nn_avgpool2_bwd(void* stream, const void* dout, void* din, int n, int 
   if (vec8({c}, {dout, din})) {
     const size_t chunks = size_t(n) * h * w * (c / 8);
     NN_LAUNCH_V(k_avgpool2_bwd_v, chunks, chunks, static_cast<const uint4*>(dout), static_cast<uint4*>(din), n, h,
-                w, c / 8, accumulate);
+                w, c / 8, accumulate, static_cast<const uint4*>(nullptr));
     NN_CHECK_LAUNCH();
   }
   k_avgpool2_bwd<<<grid1d(size_t(n) * h * w * c), 256, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -885,7 +903,7 @@ int asuna_nn_upsample2_bwd(void* stream, const void* dout, void* din, int n, int
   if (vec8({c, ctot, coff}, {dout, din})) {
     const size_t chunks = size_t(n) * 4 * h * w * (ctot / 8);
     NN_LAUNCH_V(k_upsample2_bwd_v, size_t(n) * h * w * (c / 8), chunks, static_cast<const uint4*>(dout),
-                static_cast<uint4*>(din), n, h, w, c / 8, ctot / 8, coff / 8);
+                static_cast<uint4*>(din), n, h, w, c / 8, ctot / 8, coff / 8, static_cast<const uint4*>(nullptr));
     NN_CHECK_LAUNCH();
   }
   k_upsample2_bwd<<<grid1d(size_t(n) * h * w * c), 256, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -985,6 +1003,11 @@ struct asuna_denoiser {
   int dec(int l, int k) const { return 2 * L + 2 * (L - 2 - l) + k; }
   int headIdx() const { return 4 * L - 2; }
   cudaStream_t stream() const { return ctx->stream; }
+  // Encoder level l's output over Pl pixels and its gradient: below the top
+  // level the last planes of the decoder input U, where the skip connection
+  // needs it, so that nothing is concatenated.
+  __nv_bfloat16* skip(int l, size_t Pl) const { return l == L - 1 ? lv[l].S : lv[l].U + size_t(ch[l + 1]) * Pl; }
+  __nv_bfloat16* gradSkip(int l, size_t Pl) const { return l == L - 1 ? lv[l].gS : lv[l].gU + size_t(ch[l + 1]) * Pl; }
   ~asuna_denoiser() {
     for (void* p : allocs) cudaFree(p);  // (waits for the device's work)
     if (dzReady) cudaEventDestroy(dzReady);
@@ -1015,22 +1038,63 @@ int dalloc(asuna_denoiser* d, T** p, size_t count) {
     if (rc_ != ASUNA_OK) return rc_; \
   } while (0)
 
-int convFwd(asuna_denoiser* d, int li, const __nv_bfloat16* in, int n, int h, int w, bool relu, void* out, bool f32) {
+// A layer's forward convolution, ReLU output in planes.  On tcgen05 the
+// layer's neighbours go with it: `pool` (the 2x2 mean, the next level's
+// input) and `up` (2x upsampled, the first planes of the decoder input), and
+// `out` may be null where only they are read; on mma.sync they are kernels of
+// their own.
+int convFwd(asuna_denoiser* d, int li, const __nv_bfloat16* in, int n, int h, int w, __nv_bfloat16* out,
+            __nv_bfloat16* pool, __nv_bfloat16* up) {
   const ConvLayer& c = d->layers[li];
-  if (d->useTc)
-    return asuna_nn_conv3x3_tc(d->stream(), in, n, h, w, c.cin, d->wtc + c.wtOff, d->p32 + c.bOff, c.cout,
-                               relu ? 1 : 0, nullptr, out, f32 ? 1 : 0);
-  return asuna_nn_conv3x3(d->stream(), in, n, h, w, c.cin, d->pbf + c.wOff, d->p32 + c.bOff, c.cout, relu ? 1 : 0,
-                          nullptr, out, f32 ? 1 : 0);
+  const size_t P = size_t(n) * h * w;
+  if (d->useTc) {
+    tc::Conv k;
+    k.in = in;
+    k.n = n;
+    k.h = h;
+    k.w = w;
+    k.cin = c.cin;
+    k.weights = d->wtc + c.wtOff;
+    k.bias = d->p32 + c.bOff;
+    k.cout = c.cout;
+    k.relu = true;
+    k.planes = true;
+    k.out = up && !d->training ? nullptr : out;
+    k.pool = pool;
+    k.up = up;
+    return tc::conv3x3(d->stream(), k);
+  }
+  launchConv(d->stream(), {in, d->pbf + c.wOff, d->p32 + c.bOff, nullptr, out, n, h, w, c.cin, c.cout, 1, 0,
+                           planesOf(P), planesOf(P)});
+  ASUNA_CUDA_TRY(cudaGetLastError());
+  if (pool) NN_TRY(asuna_nn_avgpool2(d->stream(), out, pool, n * (c.cout / 8), h, w, 8));
+  if (up) NN_TRY(asuna_nn_upsample2(d->stream(), out, up, n * (c.cout / 8), 2 * h, 2 * w, 8, 8, 0));
+  return ASUNA_OK;
 }
 
 // dX of layer li from dz; `mask` (the layer input's own ReLU output) fused
 int convDx(asuna_denoiser* d, int li, const __nv_bfloat16* dz, int n, int h, int w, const __nv_bfloat16* mask,
            __nv_bfloat16* dx) {
   const ConvLayer& c = d->layers[li];
-  if (d->useTc)
-    return asuna_nn_conv3x3_tc(d->stream(), dz, n, h, w, c.cout, d->wtcT + c.wtOff, nullptr, c.cin, 0, mask, dx, 0);
-  return asuna_nn_conv3x3(d->stream(), dz, n, h, w, c.cout, d->wt + c.wtOff, nullptr, c.cin, 0, mask, dx, 0);
+  const size_t P = size_t(n) * h * w;
+  if (d->useTc) {
+    tc::Conv k;
+    k.in = dz;
+    k.n = n;
+    k.h = h;
+    k.w = w;
+    k.cin = c.cout;
+    k.weights = d->wtcT + c.wtOff;
+    k.cout = c.cin;
+    k.planes = true;
+    k.mask = mask;
+    k.out = dx;
+    return tc::conv3x3(d->stream(), k);
+  }
+  launchConv(d->stream(),
+             {dz, d->wt + c.wtOff, nullptr, mask, dx, n, h, w, c.cout, c.cin, 0, 0, planesOf(P), planesOf(P)});
+  ASUNA_CUDA_TRY(cudaGetLastError());
+  return ASUNA_OK;
 }
 
 int convDw(asuna_denoiser* d, int li, const __nv_bfloat16* dz, const __nv_bfloat16* x, int n, int h, int w) {
@@ -1040,8 +1104,27 @@ int convDw(asuna_denoiser* d, int li, const __nv_bfloat16* dz, const __nv_bfloat
   const ConvLayer& c = d->layers[li];
   ASUNA_CUDA_TRY(cudaEventRecord(d->dzReady, d->stream()));
   ASUNA_CUDA_TRY(cudaStreamWaitEvent(d->side, d->dzReady, 0));
-  if (launchWgrad(d->side, dz, x, n, h, w, c.cin, c.cout, d->grad + c.wOff, d->grad + c.bOff))
+  if (launchWgrad(d->side, dz, x, n, h, w, c.cin, c.cout, d->grad + c.wOff, d->grad + c.bOff, true))
     return fail(ASUNA_ERR_CUDA, "denoiser: weight-gradient launch failed");
+  return ASUNA_OK;
+}
+
+// the gradients of pooling (added to din) and upsampling, in planes, with the
+// ReLU mask of the activation they belong to
+int poolBwd(cudaStream_t stream, const __nv_bfloat16* dout, __nv_bfloat16* din, const __nv_bfloat16* mask, int n,
+            int h, int w, int c) {
+  const size_t chunks = size_t(n) * (c / 8) * h * w;
+  NN_LAUNCH_V(k_avgpool2_bwd_v, chunks, chunks, reinterpret_cast<const uint4*>(dout), reinterpret_cast<uint4*>(din),
+              n * (c / 8), h, w, 1, 1, reinterpret_cast<const uint4*>(mask));
+  ASUNA_CUDA_TRY(cudaGetLastError());
+  return ASUNA_OK;
+}
+int upsampleBwd(cudaStream_t stream, const __nv_bfloat16* dout, __nv_bfloat16* din, const __nv_bfloat16* mask, int n,
+                int h, int w, int c) {
+  const size_t chunks = size_t(n) * (c / 8) * h * w;
+  NN_LAUNCH_V(k_upsample2_bwd_v, chunks, 4 * chunks, reinterpret_cast<const uint4*>(dout),
+              reinterpret_cast<uint4*>(din), n * (c / 8), h, w, 1, 1, 0, reinterpret_cast<const uint4*>(mask));
+  ASUNA_CUDA_TRY(cudaGetLastError());
   return ASUNA_OK;
 }
 
@@ -1078,48 +1161,62 @@ int dims(const asuna_denoiser* d, uint32_t n, uint32_t h, uint32_t w, Dims& o) {
   return ASUNA_OK;
 }
 
-// decoder input: the upsampled lower level beside the skip connection
-int upsampleConcat(cudaStream_t stream, const __nv_bfloat16* low, const __nv_bfloat16* skip, __nv_bfloat16* out, int n,
-                   int h, int w, int cu, int cs, size_t P) {
-  if (vec8({cu, cs}, {low, skip, out})) {
-    const size_t chunks = P * ((cu + cs) / 8);
-    NN_LAUNCH_V(k_upsample_concat_v, chunks, chunks, reinterpret_cast<const uint4*>(low),
-                reinterpret_cast<const uint4*>(skip), reinterpret_cast<uint4*>(out), n, h, w, cu / 8, cs / 8);
-    NN_CHECK_LAUNCH();
-  }
-  NN_TRY(asuna_nn_upsample2(stream, low, out, n, h, w, cu, cu + cs, 0));
-  return asuna_nn_copy_channels(stream, skip, cs, 0, out, cu + cs, cu, cs, P, 0);
-}
-
+// The network's output goes to `image` (h x w radiance) or, without it, to
+// d->head (the loss reads it).
 int forward(asuna_denoiser* d, const float* rad, const float* alb, const float* nrm, const float* wsum,
-            const float* noise, const Dims& D) {
+            const float* noise, const Dims& D, float4* image) {
   const int L = d->L;
   cudaStream_t s = d->stream();
   if (d->useTc) NN_TRY(flipAll(d));
   const size_t P0 = size_t(D.n) * D.hp * D.wp;
   k_prep_input<<<grid1d(P0), 256, 0, s>>>(reinterpret_cast<const float4*>(rad), reinterpret_cast<const float4*>(alb),
                                           reinterpret_cast<const float4*>(nrm), reinterpret_cast<const float4*>(wsum),
-                                          reinterpret_cast<const float4*>(noise), d->lv[0].X, D.n, D.h, D.w, D.hp,
-                                          D.wp, kInC);
+                                          reinterpret_cast<const float4*>(noise),
+                                          reinterpret_cast<uint4*>(d->lv[0].X), D.n, D.h, D.w, D.hp, D.wp);
   ASUNA_CUDA_TRY(cudaGetLastError());
   for (int l = 0; l < L; ++l) {
     const int hl = D.hp >> l, wl = D.wp >> l;
     LevelBufs& b = d->lv[l];
-    if (l > 0) NN_TRY(asuna_nn_avgpool2(s, d->lv[l - 1].S, b.X, D.n, hl * 2, wl * 2, d->ch[l - 1]));
-    NN_TRY(convFwd(d, d->enc(l, 0), b.X, D.n, hl, wl, true, b.A, false));
-    NN_TRY(convFwd(d, d->enc(l, 1), b.A, D.n, hl, wl, true, b.S, false));
+    const size_t Pl = size_t(D.n) * hl * wl;
+    NN_TRY(convFwd(d, d->enc(l, 0), b.X, D.n, hl, wl, b.A, nullptr, nullptr));
+    NN_TRY(convFwd(d, d->enc(l, 1), b.A, D.n, hl, wl, d->skip(l, Pl), l < L - 1 ? d->lv[l + 1].X : nullptr,
+                   l == L - 1 ? d->lv[l - 1].U : nullptr));
   }
   for (int l = L - 2; l >= 0; --l) {
     const int hl = D.hp >> l, wl = D.wp >> l;
-    const size_t Pl = size_t(D.n) * hl * wl;
     LevelBufs& b = d->lv[l];
-    const __nv_bfloat16* src = (l == L - 2) ? d->lv[L - 1].S : d->lv[l + 1].D;
-    const int cu = d->ch[l + 1], cs = d->ch[l], ct = cu + cs;
-    NN_TRY(upsampleConcat(s, src, b.S, b.U, D.n, hl, wl, cu, cs, Pl));
-    NN_TRY(convFwd(d, d->dec(l, 0), b.U, D.n, hl, wl, true, b.B, false));
-    NN_TRY(convFwd(d, d->dec(l, 1), b.B, D.n, hl, wl, true, b.D, false));
+    NN_TRY(convFwd(d, d->dec(l, 0), b.U, D.n, hl, wl, b.B, nullptr, nullptr));
+    NN_TRY(convFwd(d, d->dec(l, 1), b.B, D.n, hl, wl, b.D, nullptr, l > 0 ? d->lv[l - 1].U : nullptr));
   }
-  return convFwd(d, d->headIdx(), d->lv[0].D, D.n, D.hp, D.wp, false, d->head, true);
+  const ConvLayer& c = d->layers[d->headIdx()];
+  const float4* rad4 = reinterpret_cast<const float4*>(rad);
+  if (d->useTc) {
+    tc::Conv k;
+    k.in = d->lv[0].D;
+    k.n = D.n;
+    k.h = D.hp;
+    k.w = D.wp;
+    k.cin = c.cin;
+    k.weights = d->wtc + c.wtOff;
+    k.bias = d->p32 + c.bOff;
+    k.cout = c.cout;
+    k.planes = true;
+    if (image) {
+      k.image = image;
+      k.radiance = rad4;
+      k.imgH = D.h;
+      k.imgW = D.w;
+    } else {
+      k.head = reinterpret_cast<float4*>(d->head);
+    }
+    return tc::conv3x3(s, k);
+  }
+  launchConv(s, {d->lv[0].D, d->pbf + c.wOff, d->p32 + c.bOff, nullptr, d->head, D.n, D.hp, D.wp, c.cin, c.cout, 0, 1,
+                 planesOf(P0), rowsOf(c.cout)});
+  if (image)
+    k_output<<<grid1d(size_t(D.n) * D.h * D.w), 256, 0, s>>>(d->head, kHeadC, rad4, image, D.n, D.h, D.w, D.hp, D.wp);
+  ASUNA_CUDA_TRY(cudaGetLastError());
+  return ASUNA_OK;
 }
 
 int backward(asuna_denoiser* d, const Dims& D) {
@@ -1141,29 +1238,27 @@ int backward(asuna_denoiser* d, const Dims& D) {
   NN_TRY(convDx(d, d->headIdx(), d->gHead, D.n, D.hp, D.wp, d->lv[0].D, d->lv[0].gD));
   for (int l = 0; l <= L - 2; ++l) {
     const int hl = D.hp >> l, wl = D.wp >> l;
-    const size_t Pl = size_t(D.n) * hl * wl;
     LevelBufs& b = d->lv[l];
-    const int cu = d->ch[l + 1], cs = d->ch[l], ct = cu + cs;
     NN_TRY(convDw(d, d->dec(l, 1), b.gD, b.B, D.n, hl, wl));
     NN_TRY(convDx(d, d->dec(l, 1), b.gD, D.n, hl, wl, b.B, b.gB));
     NN_TRY(convDw(d, d->dec(l, 0), b.gB, b.U, D.n, hl, wl));
+    // gU's last planes are the skip connection's gradient (gradSkip)
     NN_TRY(convDx(d, d->dec(l, 0), b.gB, D.n, hl, wl, nullptr, b.gU));
-    NN_TRY(asuna_nn_copy_channels(s, b.gU, ct, cu, b.gS, cs, 0, cs, Pl, 0));
-    __nv_bfloat16* dst = (l == L - 2) ? d->lv[L - 1].gS : d->lv[l + 1].gD;
-    NN_TRY(asuna_nn_upsample2_bwd(s, b.gU, dst, D.n, hl / 2, wl / 2, cu, ct, 0));
-    if (l < L - 2) NN_TRY(asuna_nn_relu_mask(s, dst, d->lv[l + 1].D, Pl / 4 * cu));
+    const bool top = l == L - 2;
+    NN_TRY(upsampleBwd(s, b.gU, top ? d->lv[L - 1].gS : d->lv[l + 1].gD, top ? d->lv[L - 1].S : d->lv[l + 1].D, D.n,
+                       hl / 2, wl / 2, d->ch[l + 1]));
   }
   for (int l = L - 1; l >= 0; --l) {
     const int hl = D.hp >> l, wl = D.wp >> l;
     const size_t Pl = size_t(D.n) * hl * wl;
     LevelBufs& b = d->lv[l];
-    NN_TRY(asuna_nn_relu_mask(s, b.gS, b.S, Pl * d->ch[l]));
-    NN_TRY(convDw(d, d->enc(l, 1), b.gS, b.A, D.n, hl, wl));
-    NN_TRY(convDx(d, d->enc(l, 1), b.gS, D.n, hl, wl, b.A, b.gA));
+    __nv_bfloat16* gS = d->gradSkip(l, Pl);
+    NN_TRY(convDw(d, d->enc(l, 1), gS, b.A, D.n, hl, wl));
+    NN_TRY(convDx(d, d->enc(l, 1), gS, D.n, hl, wl, b.A, b.gA));
     NN_TRY(convDw(d, d->enc(l, 0), b.gA, b.X, D.n, hl, wl));
     if (l > 0) {
       NN_TRY(convDx(d, d->enc(l, 0), b.gA, D.n, hl, wl, nullptr, b.gX));
-      NN_TRY(asuna_nn_avgpool2_bwd(s, b.gX, d->lv[l - 1].gS, D.n, hl * 2, wl * 2, d->ch[l - 1], 1));
+      NN_TRY(poolBwd(s, b.gX, d->gradSkip(l - 1, 4 * Pl), d->skip(l - 1, 4 * Pl), D.n, hl * 2, wl * 2, d->ch[l - 1]));
     }
   }
   return ASUNA_OK;
@@ -1253,7 +1348,7 @@ int asuna_denoiser_create(asuna_ctx* ctx, const asuna_denoiser_opts* o, asuna_de
     const int cx = l == 0 ? kInC : d->ch[l - 1], c = d->ch[l];
     A(&b.X, Pl * cx);
     A(&b.A, Pl * c);
-    A(&b.S, Pl * c);
+    if (l == L - 1) A(&b.S, Pl * c);
     if (l <= L - 2) {
       A(&b.U, Pl * (d->ch[l + 1] + c));
       A(&b.B, Pl * c);
@@ -1262,7 +1357,7 @@ int asuna_denoiser_create(asuna_ctx* ctx, const asuna_denoiser_opts* o, asuna_de
     if (d->training) {
       if (l > 0) A(&b.gX, Pl * cx);
       A(&b.gA, Pl * c);
-      A(&b.gS, Pl * c);
+      if (l == L - 1) A(&b.gS, Pl * c);
       if (l <= L - 2) {
         A(&b.gU, Pl * (d->ch[l + 1] + c));
         A(&b.gB, Pl * c);
@@ -1270,7 +1365,7 @@ int asuna_denoiser_create(asuna_ctx* ctx, const asuna_denoiser_opts* o, asuna_de
       }
     }
   }
-  A(&d->head, size_t(o->max_pixels) * kHeadC);
+  if (d->training || !d->useTc) A(&d->head, size_t(o->max_pixels) * size_t(d->useTc ? 4 : kHeadC));
   if (d->training) A(&d->gHead, size_t(o->max_pixels) * kHeadC);
   if (rc == ASUNA_OK && d->training &&
       (cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1353,13 +1448,7 @@ int asuna_denoiser_forward(asuna_denoiser* d, const float* radiance, const float
   Dims D;
   NN_TRY(dims(d, n, h, w, D));
   ASUNA_CUDA_TRY(cudaSetDevice(d->ctx->device));
-  NN_TRY(forward(d, radiance, albedo, normal, weight, noise, D));
-  k_output<<<grid1d(size_t(n) * h * w), 256, 0, d->stream()>>>(d->head, kHeadC,
-                                                               reinterpret_cast<const float4*>(radiance),
-                                                               reinterpret_cast<float4*>(out), D.n, D.h, D.w, D.hp,
-                                                               D.wp);
-  ASUNA_CUDA_TRY(cudaGetLastError());
-  return ASUNA_OK;
+  return forward(d, radiance, albedo, normal, weight, noise, D, reinterpret_cast<float4*>(out));
 }
 
 int asuna_denoiser_loss_grad(asuna_denoiser* d, const float* radiance, const float* albedo, const float* normal,
@@ -1374,16 +1463,18 @@ int asuna_denoiser_loss_grad(asuna_denoiser* d, const float* radiance, const flo
   cudaStream_t s = d->stream();
   ASUNA_CUDA_TRY(cudaMemsetAsync(d->grad, 0, d->nParams * sizeof(float), s));
   ASUNA_CUDA_TRY(cudaMemsetAsync(d->dLoss, 0, sizeof(float), s));
-  NN_TRY(forward(d, radiance, albedo, normal, weight, noise, D));
+  NN_TRY(forward(d, radiance, albedo, normal, weight, noise, D, nullptr));
+  const int headC = d->useTc ? 4 : kHeadC;
+  uint4* gHead = reinterpret_cast<uint4*>(d->gHead);
   const size_t P0 = size_t(D.n) * D.hp * D.wp;
   const float invCount = float(1.0 / (3.0 * double(n) * h * w));
   if (d->loss == ASUNA_DENOISER_LOSS_RELMSE)
-    k_relmse_loss<<<grid1d(P0), 256, 0, s>>>(d->head, kHeadC, reinterpret_cast<const float4*>(radiance),
-                                             reinterpret_cast<const float4*>(target), d->gHead, D.n, D.h, D.w, D.hp,
+    k_relmse_loss<<<grid1d(P0), 256, 0, s>>>(d->head, headC, reinterpret_cast<const float4*>(radiance),
+                                             reinterpret_cast<const float4*>(target), gHead, D.n, D.h, D.w, D.hp,
                                              D.wp, invCount, d->dLoss);
   else
-    k_l1_loss<<<grid1d(P0), 256, 0, s>>>(d->head, kHeadC, reinterpret_cast<const float4*>(radiance),
-                                         reinterpret_cast<const float4*>(target), d->gHead, D.n, D.h, D.w, D.hp, D.wp,
+    k_l1_loss<<<grid1d(P0), 256, 0, s>>>(d->head, headC, reinterpret_cast<const float4*>(radiance),
+                                         reinterpret_cast<const float4*>(target), gHead, D.n, D.h, D.w, D.hp, D.wp,
                                          invCount, d->dLoss);
   ASUNA_CUDA_TRY(cudaGetLastError());
   NN_TRY(backward(d, D));
