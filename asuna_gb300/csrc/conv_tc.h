@@ -20,6 +20,10 @@ struct Conv {
   const void* mask = nullptr;  // out *= (mask > 0)
   void* out = nullptr;
   bool f32 = false;  // out is fp32 (rows)
+  // The grid may be launched while the stream's previous kernel still runs: it
+  // waits for that kernel's end before it touches an activation, but reads the
+  // weights and may read the bias at once (that kernel does not write them).
+  bool chained = false;
   // planes only, all of them further results; out may then be null
   void* pool = nullptr;   // the 2x2 mean of the bf16 output (h and w even)
   void* up = nullptr;     // each output pixel four times, 2h x 2w

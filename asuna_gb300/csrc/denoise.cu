@@ -1059,6 +1059,7 @@ int convFwd(asuna_denoiser* d, int li, const __nv_bfloat16* in, int n, int h, in
     k.cout = c.cout;
     k.relu = true;
     k.planes = true;
+    k.chained = true;
     k.out = up && !d->training ? nullptr : out;
     k.pool = pool;
     k.up = up;
@@ -1087,6 +1088,7 @@ int convDx(asuna_denoiser* d, int li, const __nv_bfloat16* dz, int n, int h, int
     k.weights = d->wtcT + c.wtOff;
     k.cout = c.cin;
     k.planes = true;
+    k.chained = true;
     k.mask = mask;
     k.out = dx;
     return tc::conv3x3(d->stream(), k);
@@ -1201,6 +1203,7 @@ int forward(asuna_denoiser* d, const float* rad, const float* alb, const float* 
     k.bias = d->p32 + c.bOff;
     k.cout = c.cout;
     k.planes = true;
+    k.chained = true;
     if (image) {
       k.image = image;
       k.radiance = rad4;
