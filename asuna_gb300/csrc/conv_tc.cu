@@ -97,6 +97,8 @@ uint32_t pow2Cols(int n) {
   while (c < uint32_t(n)) c <<= 1;
   return c;
 }
+}  // namespace
+
 // Output channels per CTA: the widest slice (fewest slices) that divides cout
 // into multiples of 16 and whose one-tile stages fit shared memory.
 int sliceWidth(int cout) {
@@ -106,6 +108,9 @@ int sliceWidth(int cout) {
   }
   return 16;
 }
+
+namespace {
+
 // Pixel tiles per unit (T), resident CTAs per SM, ring depth and weight
 // residency: the choice with the most tiles in flight per SM (T x CTAs),
 // where a CTA needs two accumulator buffers of T x nt tensor-memory columns

@@ -37,5 +37,8 @@ struct Conv {
 
 int conv3x3(cudaStream_t s, const Conv& c);
 
+// Output channels of a weight slice: nt in asuna_nn_weights_tc's layout.
+int sliceWidth(int cout);
+
 }  // namespace tc
 }  // namespace asuna

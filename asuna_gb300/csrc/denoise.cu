@@ -364,6 +364,55 @@ __global__ void k_flip_weights(const __nv_bfloat16* w, __nv_bfloat16* wt, int Co
   wt[(size_t(ci) * 9 + (8 - tap)) * Cout + co] = w[i];
 }
 
+// Every layer's weights in the tcgen05 operand layout, [cout/nt][cin/16][9][2]
+// [nt][8]: forward, and with `bwd` flipped and transposed for the input
+// gradient (cin and cout change places).  A thread makes one 16-byte chunk of
+// each; blockIdx.y is the layer.  (Three launches a layer took 125 us of a
+// training step; this one takes 5 us.)
+constexpr int kMaxLayers = 4 * ASUNA_DENOISER_MAX_LEVELS - 1;
+struct DeriveArgs {
+  const __nv_bfloat16* w;  // [cout][9][cin] at wOff
+  uint4 *fwd, *bwd;        // both at off (chunks)
+  struct Layer {
+    int cin, cout, nt, ntT;
+    size_t wOff, off;
+  } l[kMaxLayers];
+};
+__global__ void k_derive_weights(const __grid_constant__ DeriveArgs a) {
+  const DeriveArgs::Layer& l = a.l[blockIdx.y];
+  const int chunks = l.cout * 9 * (l.cin / 8);
+  const __nv_bfloat16* w = a.w + l.wOff;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < chunks; j += gridDim.x * blockDim.x) {
+    {
+      int r = j;
+      const int cl = r % l.nt;
+      r /= l.nt;
+      const int c = r & 1;
+      r >>= 1;
+      const int tap = r % 9;
+      r /= 9;
+      const int g = r % (l.cin / 16), slice = r / (l.cin / 16);
+      a.fwd[l.off + j] = __ldg(reinterpret_cast<const uint4*>(
+          w + (size_t(slice * l.nt + cl) * 9 + tap) * l.cin + g * 16 + c * 8));
+    }
+    if (a.bwd) {
+      int r = j;
+      const int cl = r % l.ntT;
+      r /= l.ntT;
+      const int c = r & 1;
+      r >>= 1;
+      const int tap = r % 9;
+      r /= 9;
+      const int g = r % (l.cout / 16), slice = r / (l.cout / 16);
+      const __nv_bfloat16* src = w + (size_t(g * 16 + c * 8) * 9 + (8 - tap)) * l.cin + slice * l.ntT + cl;
+      __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = src[size_t(e) * 9 * l.cin];
+      a.bwd[l.off + j] = *reinterpret_cast<const uint4*>(v);
+    }
+  }
+}
+
 __global__ void k_avgpool2(const __nv_bfloat16* in, __nv_bfloat16* out, int N, int H, int W, int C) {
   const int Ho = H / 2, Wo = W / 2;
   const size_t total = size_t(N) * Ho * Wo * C;
@@ -1099,13 +1148,17 @@ int convDx(asuna_denoiser* d, int li, const __nv_bfloat16* dz, int n, int h, int
   return ASUNA_OK;
 }
 
-int convDw(asuna_denoiser* d, int li, const __nv_bfloat16* dz, const __nv_bfloat16* x, int n, int h, int w) {
-  // on the side stream, behind what the main one has queued so far (dz): the
-  // weight gradients wait for nothing else and nothing waits for them until
-  // the step's end
-  const ConvLayer& c = d->layers[li];
+// The weight gradients run on the side stream, behind what the main one has
+// queued when sideReady is called (dz): they wait for nothing else and nothing
+// waits for them until the step's end.  One call per level: an event between
+// two of the main stream's layers keeps the second from starting early.
+int sideReady(asuna_denoiser* d) {
   ASUNA_CUDA_TRY(cudaEventRecord(d->dzReady, d->stream()));
   ASUNA_CUDA_TRY(cudaStreamWaitEvent(d->side, d->dzReady, 0));
+  return ASUNA_OK;
+}
+int convDw(asuna_denoiser* d, int li, const __nv_bfloat16* dz, const __nv_bfloat16* x, int n, int h, int w) {
+  const ConvLayer& c = d->layers[li];
   if (launchWgrad(d->side, dz, x, n, h, w, c.cin, c.cout, d->grad + c.wOff, d->grad + c.bOff, true))
     return fail(ASUNA_ERR_CUDA, "denoiser: weight-gradient launch failed");
   return ASUNA_OK;
@@ -1134,12 +1187,22 @@ int upsampleBwd(cudaStream_t stream, const __nv_bfloat16* dout, __nv_bfloat16* d
 // tcgen05 kernels, both in their operand layout
 int flipAll(asuna_denoiser* d) {
   if (d->flipped) return ASUNA_OK;
-  for (const ConvLayer& c : d->layers) {
-    NN_TRY(asuna_nn_flip_weights(d->stream(), d->pbf + c.wOff, d->wt + c.wtOff, c.cout, c.cin));
-    if (d->useTc) {
-      NN_TRY(asuna_nn_weights_tc(d->stream(), d->pbf + c.wOff, d->wtc + c.wtOff, c.cout, c.cin));
-      NN_TRY(asuna_nn_weights_tc(d->stream(), d->wt + c.wtOff, d->wtcT + c.wtOff, c.cin, c.cout));
+  if (d->useTc) {
+    DeriveArgs a{};
+    a.w = d->pbf;
+    a.fwd = reinterpret_cast<uint4*>(d->wtc);
+    a.bwd = reinterpret_cast<uint4*>(d->wtcT);
+    int most = 1;
+    for (size_t i = 0; i < d->layers.size(); ++i) {
+      const ConvLayer& c = d->layers[i];
+      a.l[i] = {c.cin, c.cout, tc::sliceWidth(c.cout), tc::sliceWidth(c.cin), c.wOff, c.wtOff / 8};
+      most = std::max(most, c.cout * 9 * (c.cin / 8));
     }
+    k_derive_weights<<<dim3((most + 255) / 256, unsigned(d->layers.size())), 256, 0, d->stream()>>>(a);
+    ASUNA_CUDA_TRY(cudaGetLastError());
+  } else {
+    for (const ConvLayer& c : d->layers)
+      NN_TRY(asuna_nn_flip_weights(d->stream(), d->pbf + c.wOff, d->wt + c.wtOff, c.cout, c.cin));
   }
   d->flipped = true;
   return ASUNA_OK;
@@ -1237,16 +1300,18 @@ int backward(asuna_denoiser* d, const Dims& D) {
       }
     }
   } join{d};
+  NN_TRY(sideReady(d));
   NN_TRY(convDw(d, d->headIdx(), d->gHead, d->lv[0].D, D.n, D.hp, D.wp));
   NN_TRY(convDx(d, d->headIdx(), d->gHead, D.n, D.hp, D.wp, d->lv[0].D, d->lv[0].gD));
   for (int l = 0; l <= L - 2; ++l) {
     const int hl = D.hp >> l, wl = D.wp >> l;
     LevelBufs& b = d->lv[l];
-    NN_TRY(convDw(d, d->dec(l, 1), b.gD, b.B, D.n, hl, wl));
     NN_TRY(convDx(d, d->dec(l, 1), b.gD, D.n, hl, wl, b.B, b.gB));
-    NN_TRY(convDw(d, d->dec(l, 0), b.gB, b.U, D.n, hl, wl));
     // gU's last planes are the skip connection's gradient (gradSkip)
     NN_TRY(convDx(d, d->dec(l, 0), b.gB, D.n, hl, wl, nullptr, b.gU));
+    NN_TRY(sideReady(d));
+    NN_TRY(convDw(d, d->dec(l, 1), b.gD, b.B, D.n, hl, wl));
+    NN_TRY(convDw(d, d->dec(l, 0), b.gB, b.U, D.n, hl, wl));
     const bool top = l == L - 2;
     NN_TRY(upsampleBwd(s, b.gU, top ? d->lv[L - 1].gS : d->lv[l + 1].gD, top ? d->lv[L - 1].S : d->lv[l + 1].D, D.n,
                        hl / 2, wl / 2, d->ch[l + 1]));
@@ -1256,13 +1321,13 @@ int backward(asuna_denoiser* d, const Dims& D) {
     const size_t Pl = size_t(D.n) * hl * wl;
     LevelBufs& b = d->lv[l];
     __nv_bfloat16* gS = d->gradSkip(l, Pl);
-    NN_TRY(convDw(d, d->enc(l, 1), gS, b.A, D.n, hl, wl));
     NN_TRY(convDx(d, d->enc(l, 1), gS, D.n, hl, wl, b.A, b.gA));
+    if (l > 0) NN_TRY(convDx(d, d->enc(l, 0), b.gA, D.n, hl, wl, nullptr, b.gX));
+    NN_TRY(sideReady(d));
+    NN_TRY(convDw(d, d->enc(l, 1), gS, b.A, D.n, hl, wl));
     NN_TRY(convDw(d, d->enc(l, 0), b.gA, b.X, D.n, hl, wl));
-    if (l > 0) {
-      NN_TRY(convDx(d, d->enc(l, 0), b.gA, D.n, hl, wl, nullptr, b.gX));
+    if (l > 0)
       NN_TRY(poolBwd(s, b.gX, d->gradSkip(l - 1, 4 * Pl), d->skip(l - 1, 4 * Pl), D.n, hl * 2, wl * 2, d->ch[l - 1]));
-    }
   }
   return ASUNA_OK;
 }
@@ -1332,10 +1397,11 @@ int asuna_denoiser_create(asuna_ctx* ctx, const asuna_denoiser_opts* o, asuna_de
   };
   A(&d->p32, d->nParams);
   A(&d->pbf, d->nParams);
-  A(&d->wt, d->nFlip);
   if (d->useTc) {
     A(&d->wtc, d->nFlip);
-    A(&d->wtcT, d->nFlip);
+    if (d->training) A(&d->wtcT, d->nFlip);
+  } else {
+    A(&d->wt, d->nFlip);
   }
   A(&d->dLoss, 1);
   A(&d->dSums, 8);

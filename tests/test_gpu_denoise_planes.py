@@ -53,3 +53,26 @@ def test_fused_layers(dctx, ch, shape):
         assert np.median(np.abs(got - ro) / (np.abs(ro) + 1e-3)) < 5e-3
         assert np.abs(got - ro).max() <= 0.05 * np.abs(ro).max()
         assert np.all(outs[False, tm][..., 3] == 1.0)
+
+
+@pytest.mark.parametrize("ch", [(16, 16), (32, 256), (48, 64, 192)])
+def test_gradients_with_sliced_weights(dctx, ch):
+    """Loss and gradients on tcgen05 against mma.sync, where layers have one
+    and several weight slices in either direction."""
+    n, h, w = 2, 19, 26
+    rng = np.random.default_rng(sum(ch))
+    rad = rng.gamma(1.2, 0.5, (n, h, w, 4)).astype(np.float32)
+    tgt = (rad * rng.uniform(0.5, 1.5, rad.shape)).astype(np.float32)
+    p = U.he_init(ch, 6)
+    p = (p + rng.normal(0, 0.02, p.size)).astype(np.float32)
+    res = []
+    for tm in (False, True):
+        d = dn.Denoiser(dctx, ch, seed=3, max_pixels=n * 32 * 32, training=True, tensor_memory=tm)
+        d.set_params(p)
+        grad, gtgt = torch.from_numpy(rad).cuda(), torch.from_numpy(tgt).cuda()
+        torch.cuda.synchronize()
+        res.append((d.loss_grad(grad, None, None, None, gtgt), d.get_grads().astype(np.float64)))
+    (l0, g0), (l1, g1) = res
+    # bounds as for the default network: accumulation order before bf16 rounding
+    assert abs(l1 - l0) <= 1e-3 * l0
+    assert np.linalg.norm(g1 - g0) < 0.03 * np.linalg.norm(g0)
