@@ -90,13 +90,11 @@ struct BuildCtx {
   uint32_t* ordFinal;
   BvhNode* nodes;
   uint32_t nodeCap;
-  uint32_t* counters;  // [0] nodes used, [1] max depth, [2] error, [3] next-level large tasks, [4] small tasks
-  BTask* nextLarge;
-  uint32_t nextLargeCap;
+  uint32_t* counters;  // kCtr*
   BTask* small;
   uint32_t smallCap;
 };
-enum { kCtrNodes = 0, kCtrDepth = 1, kCtrError = 2, kCtrNextLarge = 3, kCtrSmall = 4, kCtrSmallNext = 5, kCtrNum = 8 };
+enum { kCtrNodes = 0, kCtrDepth = 1, kCtrError = 2, kCtrSmall = 3, kCtrSmallNext = 4, kCtrNum = 8 };
 enum { kErrNodes = 1, kErrStack = 2, kErrTasks = 4 };
 
 __device__ __forceinline__ float boxArea(float lx, float ly, float lz, float hx, float hy, float hz) {
@@ -428,11 +426,31 @@ struct Chunk {
   uint32_t task, first, last;
 };
 
-__global__ void __launch_bounds__(256) k_binLarge(BuildCtx C, const BTask* __restrict__ tasks,
-                                                  const Chunk* __restrict__ chunks, uint32_t* gbins) {
+// One level of large tasks.  The tasks, their chunks and their numbers are
+// made on the device by the level before (k_childrenLarge), so that the host
+// issues levels without waiting for any; a launch covers the most there can be
+// (LargeCtx's bounds) and what is beyond the numbers, or follows an error,
+// returns at once.
+struct LargeCtx {
+  const BTask* tasks;
+  const uint32_t* count;  // [0] tasks, [1] chunks
+  Chunk* chunks;
+  uint32_t taskCap, chunkCap;
+  uint32_t* gbins;  // [taskCap][kTaskBinWords], all initial between levels
+  BSplit* splits;
+  uint32_t* cursors;
+  BTask* next;
+  uint32_t* nextCount;
+  __device__ __forceinline__ bool has(const BuildCtx& C, uint32_t i, int what) const {
+    return i < min(count[what], what ? chunkCap : taskCap) && C.counters[kCtrError] == 0u;
+  }
+};
+
+__global__ void __launch_bounds__(256) k_binLarge(BuildCtx C, LargeCtx L) {
   __shared__ uint32_t bins[kTaskBinWords];
-  const Chunk ch = chunks[blockIdx.x];
-  const BTask t = tasks[ch.task];
+  if (!L.has(C, blockIdx.x, 1)) return;
+  const Chunk ch = L.chunks[blockIdx.x];
+  const BTask t = L.tasks[ch.task];
   clearBins(bins, threadIdx.x, blockDim.x);
   __syncthreads();
   float scale[3];
@@ -440,7 +458,7 @@ __global__ void __launch_bounds__(256) k_binLarge(BuildCtx C, const BTask* __res
   const uint32_t* ord = C.ord[taskBuf(t)];
   for (uint32_t i = ch.first + threadIdx.x; i < ch.last; i += blockDim.x) binPrim(bins, C, ord[i], t.clo, scale);
   __syncthreads();
-  uint32_t* g = gbins + size_t(ch.task) * kTaskBinWords;
+  uint32_t* g = L.gbins + size_t(ch.task) * kTaskBinWords;
   for (int i = threadIdx.x; i < kTaskBinWords; i += blockDim.x) {
     const int w = i % kBinWords;
     const uint32_t v = bins[i];
@@ -455,19 +473,21 @@ __global__ void __launch_bounds__(256) k_binLarge(BuildCtx C, const BTask* __res
 }
 
 __global__ void k_clearBins(uint32_t* gbins, uint32_t ntasks) {
-  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= size_t(ntasks) * kTaskBinWords) return;
-  gbins[i] = initWord(int(i % kBinWords));
+  const size_t n = size_t(ntasks) * kTaskBinWords;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+    gbins[i] = initWord(int(i % kBinWords));
 }
 
-// One warp per large task: the split, the inner node, the partition cursors.
-__global__ void k_splitLarge(BuildCtx C, const BTask* __restrict__ tasks, uint32_t ntasks,
-                             const uint32_t* __restrict__ gbins, BSplit* splits, uint32_t* cursors) {
+__global__ void k_splitLarge(BuildCtx C, LargeCtx L) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
   const int lane = threadIdx.x & 31;
-  if (w >= ntasks) return;
-  const BTask t = tasks[w];
-  BSplit s = decideSplit(gbins + size_t(w) * kTaskBinWords, t, lane);
+  // (one answer for the warp: another may record an error meanwhile)
+  if (!__shfl_sync(0xffffffffu, int(L.has(C, w, 0)), 0)) return;
+  const BTask t = L.tasks[w];
+  uint32_t* bins = L.gbins + size_t(w) * kTaskBinWords;
+  BSplit s = decideSplit(bins, t, lane);
+  __syncwarp();
+  clearBins(bins, lane, 32);  // for the next level
   if (lane == 0) {
     noteDepth(C, taskDepth(t));
     // large tasks always hold more primitives than a leaf: kind 0 cannot occur
@@ -484,19 +504,22 @@ __global__ void k_splitLarge(BuildCtx C, const BTask* __restrict__ tasks, uint32
       return int32_t(i);
     });
     s.node = node;
-    splits[w] = s;
-    cursors[2 * w] = t.begin;
-    cursors[2 * w + 1] = t.begin + s.nL;
+    L.splits[w] = s;
+    L.cursors[2 * w] = t.begin;
+    L.cursors[2 * w + 1] = t.begin + s.nL;
   }
 }
 
-__global__ void __launch_bounds__(256) k_partitionLarge(BuildCtx C, const BTask* __restrict__ tasks,
-                                                        const Chunk* __restrict__ chunks,
-                                                        const BSplit* __restrict__ splits, uint32_t* cursors) {
+__global__ void __launch_bounds__(256) k_partitionLarge(BuildCtx C, LargeCtx L) {
   __shared__ uint32_t warpL[8], warpR[8], baseL, baseR;
-  const Chunk ch = chunks[blockIdx.x];
-  const BTask t = tasks[ch.task];
-  const BSplit& s = splits[ch.task];
+  __shared__ bool on;  // (another block may record an error meanwhile)
+  if (threadIdx.x == 0) on = L.has(C, blockIdx.x, 1);
+  __syncthreads();
+  if (!on) return;
+  const Chunk ch = L.chunks[blockIdx.x];
+  const BTask t = L.tasks[ch.task];
+  const BSplit& s = L.splits[ch.task];
+  uint32_t* cursors = L.cursors;
   const uint32_t* src = C.ord[taskBuf(t)];
   uint32_t* dst = C.ord[taskBuf(t) ^ 1u];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x / 32u;
@@ -539,12 +562,14 @@ __global__ void __launch_bounds__(256) k_partitionLarge(BuildCtx C, const BTask*
 }
 
 // Child tasks of the large tasks: to the next level, or to the small list.
-__global__ void k_childrenLarge(BuildCtx C, const BTask* __restrict__ tasks, uint32_t ntasks,
-                                const BSplit* __restrict__ splits) {
+// Chunks [f, f + kChunk) of task i, appended to a level's list.
+__host__ __device__ __forceinline__ uint32_t chunksOf(uint32_t prims) { return (prims + kChunk - 1) / kChunk; }
+
+__global__ void k_childrenLarge(BuildCtx C, LargeCtx L) {
   const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= ntasks) return;
-  const BTask t = tasks[w];
-  const BSplit s = splits[w];
+  if (!L.has(C, w, 0)) return;
+  const BTask t = L.tasks[w];
+  const BSplit s = L.splits[w];
   if (s.node < 0) return;
   BTask ch[2];
   childTasks(t, s, s.node, ch[0], ch[1]);
@@ -563,9 +588,14 @@ __global__ void k_childrenLarge(BuildCtx C, const BTask* __restrict__ tasks, uin
     }
     const uint32_t n = c.end - c.begin;
     if (n > kSmallTask) {
-      const uint32_t i = atomicAdd(&C.counters[kCtrNextLarge], 1u);
-      if (i < C.nextLargeCap) C.nextLarge[i] = c;
-      else atomicOr(&C.counters[kCtrError], uint32_t(kErrTasks));
+      const uint32_t nc = chunksOf(n), i = atomicAdd(&L.nextCount[0], 1u), b = atomicAdd(&L.nextCount[1], nc);
+      if (i < L.taskCap && b + nc <= L.chunkCap) {
+        L.next[i] = c;
+        for (uint32_t k2 = 0; k2 < nc; ++k2)
+          L.chunks[b + k2] = {i, c.begin + k2 * kChunk, min(c.end, c.begin + (k2 + 1) * kChunk)};
+      } else {
+        atomicOr(&C.counters[kCtrError], uint32_t(kErrTasks));
+      }
     } else {
       const uint32_t i = atomicAdd(&C.counters[kCtrSmall], 1u);
       if (i < C.smallCap) C.small[i] = c;
@@ -937,13 +967,23 @@ __global__ void k_checkOrder(const uint32_t* __restrict__ triBase, int nm, uint3
   if (atomicExch(&seen[p], 1u) != 0u) atomicAdd(errors, 1u);
 }
 
-template <class T>
-int devAlloc(T** p, size_t n, std::vector<void*>& tmp) {
-  *p = nullptr;
-  ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)));
-  tmp.push_back(*p);
-  return ASUNA_OK;
-}
+// The build's temporary arrays, in one allocation (an allocation and its
+// release take 60 to 120 us whatever their size, and there are eighteen).
+struct Scratch {
+  unsigned char* base = nullptr;
+  size_t size = 0;
+  ~Scratch() { cudaFree(base); }
+  template <class T>
+  size_t add(size_t n) {
+    const size_t at = size;
+    size += (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+    return at;
+  }
+  template <class T>
+  T* get(size_t at) const {
+    return reinterpret_cast<T*>(base + at);
+  }
+};
 
 }  // namespace
 
@@ -953,13 +993,6 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
   const uint32_t N = triBase[nm];
   out = DeviceBlas{};
   out.roots.assign(nm, -1);
-  std::vector<void*> tmp;
-  struct Free {
-    std::vector<void*>& v;
-    ~Free() {
-      for (void* p : v) cudaFree(p);
-    }
-  } freeTmp{tmp};
   // small tasks: the leaves of the binary tree of large tasks, of which a
   // level has at most N / kSmallTask and there are at most kMedianDepth levels
   // of SAH splits (however lopsided) and then 32 of halvings
@@ -978,17 +1011,32 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
   const uint32_t nodeCap = uint32_t(cap64);
   ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&out.nodes), size_t(nodeCap + extraNodes) * sizeof(BvhNode)));
   ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&out.tris), std::max<size_t>(N, 1) * sizeof(TriDev)));
-  out.nodeCapacity = nodeCap + extraNodes;
   if (N == 0) return ASUNA_OK;
 
-  uint32_t *dTriBase, *dVtxBase, *meshKeys, *counters, *ordFinal, *ord0, *ord1;
-  float4 *pbox, *cen;
-  int rc;
-  if ((rc = devAlloc(&dTriBase, nm + 1, tmp)) || (rc = devAlloc(&dVtxBase, nm, tmp)) ||
-      (rc = devAlloc(&meshKeys, size_t(nm) * 12, tmp)) || (rc = devAlloc(&counters, kCtrNum, tmp)) ||
-      (rc = devAlloc(&ordFinal, N, tmp)) || (rc = devAlloc(&ord0, N, tmp)) || (rc = devAlloc(&ord1, N, tmp)) ||
-      (rc = devAlloc(&pbox, size_t(N) * 2, tmp)) || (rc = devAlloc(&cen, N, tmp)))
-    return rc;
+  // a level's large tasks are disjoint and hold more than kSmallTask primitives
+  const uint32_t taskCap = N / kSmallTask + 1, chunkCap = N / kChunk + taskCap + 1;
+  constexpr uint32_t kLevels = kMedianDepth + 32;
+  Scratch scratch;
+  const size_t oTriBase = scratch.add<uint32_t>(nm + 1), oVtxBase = scratch.add<uint32_t>(nm),
+               oKeys = scratch.add<uint32_t>(size_t(nm) * 12), oCounters = scratch.add<uint32_t>(kCtrNum),
+               oLevels = scratch.add<uint32_t>(2 * (kLevels + 1)), oOrdFinal = scratch.add<uint32_t>(N),
+               oOrd0 = scratch.add<uint32_t>(N), oOrd1 = scratch.add<uint32_t>(N),
+               oPbox = scratch.add<float4>(size_t(N) * 2), oCen = scratch.add<float4>(N),
+               oTasks0 = scratch.add<BTask>(taskCap), oTasks1 = scratch.add<BTask>(taskCap),
+               oSmall = scratch.add<BTask>(smallMax), oChunks = scratch.add<Chunk>(chunkCap),
+               oBins = scratch.add<uint32_t>(size_t(taskCap) * kTaskBinWords),
+               oSplits = scratch.add<BSplit>(taskCap), oCursors = scratch.add<uint32_t>(size_t(taskCap) * 2),
+               oSeen = scratch.add<uint32_t>(size_t(N) + 1);
+  ASUNA_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&scratch.base), scratch.size));
+  uint32_t *const dTriBase = scratch.get<uint32_t>(oTriBase), *const dVtxBase = scratch.get<uint32_t>(oVtxBase),
+                  *const meshKeys = scratch.get<uint32_t>(oKeys), *const counters = scratch.get<uint32_t>(oCounters),
+                  *const levelCounts = scratch.get<uint32_t>(oLevels),
+                  *const ordFinal = scratch.get<uint32_t>(oOrdFinal), *const ord0 = scratch.get<uint32_t>(oOrd0),
+                  *const ord1 = scratch.get<uint32_t>(oOrd1);
+  float4 *const pbox = scratch.get<float4>(oPbox), *const cen = scratch.get<float4>(oCen);
+  BTask* const dTasks[2] = {scratch.get<BTask>(oTasks0), scratch.get<BTask>(oTasks1)};
+  BTask* const dSmall = scratch.get<BTask>(oSmall);
+  Chunk* const dChunks = scratch.get<Chunk>(oChunks);
   ASUNA_CUDA_TRY(cudaMemcpyAsync(dTriBase, triBase.data(), (nm + 1) * 4, cudaMemcpyHostToDevice, st));
   ASUNA_CUDA_TRY(cudaMemcpyAsync(dVtxBase, vtxBase.data(), nm * 4, cudaMemcpyHostToDevice, st));
   {
@@ -1041,12 +1089,6 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
     const uint32_t c0 = nroots;
     ASUNA_CUDA_TRY(cudaMemcpyAsync(&counters[kCtrNodes], &c0, 4, cudaMemcpyHostToDevice, st));
   }
-  // task lists
-  BTask *dLarge, *dNext, *dSmall;
-  const uint32_t largeCap = 2 * (N / kSmallTask + 1) + uint32_t(nm) + 16;
-  if ((rc = devAlloc(&dLarge, largeCap, tmp)) || (rc = devAlloc(&dNext, largeCap, tmp)) ||
-      (rc = devAlloc(&dSmall, smallMax, tmp)))
-    return rc;
   if (smallInit.size() > smallMax) return fail(ASUNA_ERR_INVALID, "device BVH build: too many small meshes");
   if (!smallInit.empty())
     ASUNA_CUDA_TRY(cudaMemcpyAsync(dSmall, smallInit.data(), smallInit.size() * sizeof(BTask), cudaMemcpyHostToDevice,
@@ -1064,68 +1106,67 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
   C.nodes = out.nodes;
   C.nodeCap = nodeCap;
   C.counters = counters;
-  C.nextLarge = dNext;
-  C.nextLargeCap = largeCap;
   C.small = dSmall;
   C.smallCap = smallMax;
   // ---- large tasks, level by level ----
-  uint32_t* gbins = nullptr;
-  BSplit* splits = nullptr;
-  uint32_t* cursors = nullptr;
-  Chunk* dChunks = nullptr;
-  size_t gbinsCap = 0, chunksCap = 0;
-  int levels = 0;
-  while (!large.empty()) {
-    if (++levels > int(kMedianDepth) + 32) return fail(ASUNA_ERR_INVALID, "device BVH build: no progress");
-    const uint32_t nt = uint32_t(large.size());
+  uint32_t ctr[kCtrNum] = {};
+  ctr[kCtrSmall] = uint32_t(smallInit.size());
+  if (!large.empty()) {
+    // The levels that the largest mesh needs when its halves are even, and
+    // one, are issued at once; then the host looks, and goes on two at a time
+    // (scene creation at 2M triangles, 9 levels of two looks and four copies
+    // before: 7.5 -> 6.0 ms, with the one allocation; at 21M 44.6 -> 41.0).
     std::vector<Chunk> chunks;
-    for (uint32_t t = 0; t < nt; ++t)
-      for (uint32_t f = large[t].begin; f < large[t].end; f += kChunk)
-        chunks.push_back({t, f, std::min(large[t].end, f + kChunk)});
-    if (nt > gbinsCap) {
-      if (gbins) cudaFree(gbins);
-      if (splits) cudaFree(splits);
-      if (cursors) cudaFree(cursors);
-      tmp.erase(std::remove_if(tmp.begin(), tmp.end(),
-                               [&](void* p) { return p == gbins || p == splits || p == cursors; }),
-                tmp.end());
-      gbinsCap = std::max<size_t>(nt, 64);
-      if ((rc = devAlloc(&gbins, gbinsCap * kTaskBinWords, tmp)) || (rc = devAlloc(&splits, gbinsCap, tmp)) ||
-          (rc = devAlloc(&cursors, gbinsCap * 2, tmp)))
-        return rc;
+    uint32_t most = 0;
+    for (uint32_t t = 0; t < large.size(); ++t) {
+      const uint32_t n = large[t].end - large[t].begin;
+      most = std::max(most, n);
+      for (uint32_t k = 0; k < chunksOf(n); ++k)
+        chunks.push_back({t, large[t].begin + k * kChunk, std::min(large[t].end, large[t].begin + (k + 1) * kChunk)});
     }
-    if (chunks.size() > chunksCap) {
-      if (dChunks) cudaFree(dChunks);
-      tmp.erase(std::remove(tmp.begin(), tmp.end(), static_cast<void*>(dChunks)), tmp.end());
-      chunksCap = std::max<size_t>(chunks.size(), 256);
-      if ((rc = devAlloc(&dChunks, chunksCap, tmp))) return rc;
-    }
-    ASUNA_CUDA_TRY(cudaMemcpyAsync(dLarge, large.data(), nt * sizeof(BTask), cudaMemcpyHostToDevice, st));
+    const uint32_t first[2] = {uint32_t(large.size()), uint32_t(chunks.size())};
+    if (first[0] > taskCap || first[1] > chunkCap) return fail(ASUNA_ERR_INVALID, "device BVH build: too many tasks");
+    ASUNA_CUDA_TRY(cudaMemsetAsync(levelCounts, 0, 2 * (kLevels + 1) * sizeof(uint32_t), st));
+    ASUNA_CUDA_TRY(cudaMemcpyAsync(levelCounts, first, sizeof(first), cudaMemcpyHostToDevice, st));
+    ASUNA_CUDA_TRY(
+        cudaMemcpyAsync(dTasks[0], large.data(), large.size() * sizeof(BTask), cudaMemcpyHostToDevice, st));
     ASUNA_CUDA_TRY(
         cudaMemcpyAsync(dChunks, chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-    const size_t nb = size_t(nt) * kTaskBinWords;
-    k_clearBins<<<unsigned((nb + 255) / 256), 256, 0, st>>>(gbins, nt);
-    k_binLarge<<<unsigned(chunks.size()), 256, 0, st>>>(C, dLarge, dChunks, gbins);
-    k_splitLarge<<<(nt * 32 + 127) / 128, 128, 0, st>>>(C, dLarge, nt, gbins, splits, cursors);
-    k_partitionLarge<<<unsigned(chunks.size()), 256, 0, st>>>(C, dLarge, dChunks, splits, cursors);
-    const uint32_t zero = 0;
-    ASUNA_CUDA_TRY(cudaMemcpyAsync(&counters[kCtrNextLarge], &zero, 4, cudaMemcpyHostToDevice, st));
-    k_childrenLarge<<<(nt + 127) / 128, 128, 0, st>>>(C, dLarge, nt, splits);
-    ASUNA_CUDA_TRY(cudaGetLastError());
-    uint32_t ctr[kCtrNum];
-    ASUNA_CUDA_TRY(cudaMemcpyAsync(ctr, counters, sizeof(ctr), cudaMemcpyDeviceToHost, st));
-    ASUNA_CUDA_TRY(cudaStreamSynchronize(st));
-    if (ctr[kCtrError]) return fail(ASUNA_ERR_INVALID, "device BVH build failed (error bits %u)", ctr[kCtrError]);
-    const uint32_t nn = std::min(ctr[kCtrNextLarge], largeCap);
-    large.resize(nn);
-    if (nn)
-      ASUNA_CUDA_TRY(cudaMemcpyAsync(large.data(), dNext, nn * sizeof(BTask), cudaMemcpyDeviceToHost, st));
-    ASUNA_CUDA_TRY(cudaStreamSynchronize(st));
+    LargeCtx L;
+    L.chunks = dChunks;
+    L.taskCap = taskCap;
+    L.chunkCap = chunkCap;
+    L.gbins = scratch.get<uint32_t>(oBins);
+    L.splits = scratch.get<BSplit>(oSplits);
+    L.cursors = scratch.get<uint32_t>(oCursors);
+    k_clearBins<<<unsigned(sms) * 8, 256, 0, st>>>(L.gbins, taskCap);
+    uint32_t batch = 1;
+    for (uint32_t n = most; n > kSmallTask; n = (n + 1) / 2) ++batch;
+    uint64_t tasks = first[0];  // at most, on this level
+    for (uint32_t level = 0, left = 1; left;) {
+      if (level == kLevels) return fail(ASUNA_ERR_INVALID, "device BVH build: no progress");
+      for (const uint32_t end = std::min(level + batch, kLevels); level < end; ++level) {
+        const unsigned nt = unsigned(std::min<uint64_t>(tasks, taskCap));
+        const unsigned nc = std::min(chunkCap, N / kChunk + nt);
+        L.tasks = dTasks[level & 1u];
+        L.next = dTasks[(level & 1u) ^ 1u];
+        L.count = levelCounts + 2 * level;
+        L.nextCount = levelCounts + 2 * (level + 1);
+        k_binLarge<<<nc, 256, 0, st>>>(C, L);
+        k_splitLarge<<<(nt * 32 + 127) / 128, 128, 0, st>>>(C, L);
+        k_partitionLarge<<<nc, 256, 0, st>>>(C, L);
+        k_childrenLarge<<<(nt + 127) / 128, 128, 0, st>>>(C, L);
+        tasks = std::min<uint64_t>(2 * tasks, taskCap);
+      }
+      ASUNA_CUDA_TRY(cudaGetLastError());
+      ASUNA_CUDA_TRY(cudaMemcpyAsync(&left, levelCounts + 2 * level, 4, cudaMemcpyDeviceToHost, st));
+      ASUNA_CUDA_TRY(cudaMemcpyAsync(ctr, counters, sizeof(ctr), cudaMemcpyDeviceToHost, st));
+      ASUNA_CUDA_TRY(cudaStreamSynchronize(st));
+      if (ctr[kCtrError]) return fail(ASUNA_ERR_INVALID, "device BVH build failed (error bits %u)", ctr[kCtrError]);
+      batch = 2;
+    }
   }
   // ---- small tasks: one warp per subtree ----
-  uint32_t ctr[kCtrNum];
-  ASUNA_CUDA_TRY(cudaMemcpyAsync(ctr, counters, sizeof(ctr), cudaMemcpyDeviceToHost, st));
-  ASUNA_CUDA_TRY(cudaStreamSynchronize(st));
   const uint32_t nsmall = std::min(ctr[kCtrSmall], smallMax);
   if (nsmall) {
     const uint32_t grid = std::max(1u, std::min(smallGrid, (nsmall + kSmallWarps - 1) / kSmallWarps));
@@ -1133,8 +1174,7 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
     ASUNA_CUDA_TRY(cudaGetLastError());
   }
   // ---- leaf triangles ----
-  uint32_t* seen;
-  if ((rc = devAlloc(&seen, N + 1, tmp))) return rc;
+  uint32_t* const seen = scratch.get<uint32_t>(oSeen);
   ASUNA_CUDA_TRY(cudaMemsetAsync(seen, 0, size_t(N + 1) * 4, st));
   k_checkOrder<<<(N + 255) / 256, 256, 0, st>>>(dTriBase, nm, N, ordFinal, seen, seen + N);
   k_emitTris<<<(N + 255) / 256, 256, 0, st>>>(vtx, idx, dTriBase, dVtxBase, nm, N, ordFinal, out.tris);
@@ -1150,22 +1190,6 @@ int buildBlasDevice(const VtxDev* vtx, const uint4* idx, const std::vector<uint3
   out.rootNodes.resize(nroots);
   if (nroots)
     ASUNA_CUDA_TRY(cudaMemcpy(out.rootNodes.data(), out.nodes, nroots * sizeof(BvhNode), cudaMemcpyDeviceToHost));
-  // the capacity bound is loose (about one node per primitive): move the
-  // nodes into an array of the size used, with the caller's extra room
-  const size_t used = size_t(out.nodeCount) + extraNodes;
-  if (used < size_t(out.nodeCapacity) * 9 / 10) {
-    BvhNode* tight = nullptr;
-    if (cudaMalloc(reinterpret_cast<void**>(&tight), used * sizeof(BvhNode)) == cudaSuccess) {
-      ASUNA_CUDA_TRY(cudaMemcpyAsync(tight, out.nodes, size_t(out.nodeCount) * sizeof(BvhNode),
-                                     cudaMemcpyDeviceToDevice, st));
-      ASUNA_CUDA_TRY(cudaStreamSynchronize(st));
-      cudaFree(out.nodes);
-      out.nodes = tight;
-      out.nodeCapacity = uint32_t(used);
-    } else {
-      cudaGetLastError();  // keep the loose array
-    }
-  }
   return ASUNA_OK;
 }
 

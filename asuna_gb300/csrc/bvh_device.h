@@ -14,7 +14,6 @@ struct DeviceBlas {
   BvhNode* nodes = nullptr;        // device; BLAS nodes first, room for `extraNodes` more after them
   TriDev* tris = nullptr;          // device; leaf order, triBase[m] + i for mesh m
   uint32_t nodeCount = 0;          // BLAS node slots used (unused chunk tails included)
-  uint32_t nodeCapacity = 0;
   uint32_t maxDepth = 0;           // deepest task (root = 1)
   std::vector<int32_t> roots;      // per mesh: root node (-1: no triangles)
   std::vector<BvhNode> rootNodes;  // host copies of the root nodes, in root order
