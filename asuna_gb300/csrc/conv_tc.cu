@@ -37,7 +37,7 @@
 // copies, pooling and output kernels; the convolutions themselves take 757 ->
 // 652 us with those in them, as planes load and store whole lines).
 //
-// Four CTAs per SM (80 registers a thread) are what hides one tile's epilogue
+// Four CTAs per SM (at most 80 registers a thread) are what hides one tile's epilogue
 // behind the others' copies and MMAs: at 118 registers, two CTAs, the image
 // took 930 us instead of 752.  The network's layers are chained: a layer's CTAs
 // are launched, allocate, load their first weights and bias while the previous
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
   const int S = a.stages;
   unsigned char* actBase = sm + headerBytes(a.nt);
   unsigned char* wBase = actBase + S * stageA;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
   // for that before they touch either; the weights were there before (a grid
   // launched alone waits for nothing).
   auto waitForPrevious = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
-  const uint32_t tmem = *tmemSlot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmemSlot, 0);
   const int groups = a.cin / 16;
   const int myUnits = blockIdx.x < a.units ? (a.units - 1 - int(blockIdx.x)) / int(gridDim.x) + 1 : 0;
   const int total = myUnits * groups;  // stream position q = (unit k of this CTA, channel group g)
@@ -446,34 +446,33 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
       if (a.resident && total > 0) mbarWaitOr(smem(wFull), 0u, &kNeverAbort);
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
-      if (!*abortFlag) {
-        const uint32_t idesc = instrDesc(uint32_t(a.nt));
-        const uint32_t bTap = uint32_t(2 * a.nt);  // (16-byte units)
-        const uint64_t da0 = matDesc(smem(actBase), chunk, uint32_t(hw * 16));
-        const uint64_t db0 = matDesc(smem(wBase), uint32_t(a.nt * 16), 128u);
-        bool ok = !a.resident || total == 0 || mbarWaitOr(smem(wFull), 0u, abortFlag);
-        if (!ok) fail();
-        int k = 0, g = 0, s = 0;
-        uint32_t use = 0;
-        for (int q = 0; q < total && ok; ++q) {
-          const uint32_t buf = uint32_t(k & 1);
-          if (g == 0 && k >= 2) {
-            // the epilogue has read this buffer's previous unit out
-            if (!mbarWaitOr(smem(&accEmpty[buf]), uint32_t((k >> 1) - 1) & 1u, abortFlag)) {
-              fail();
-              break;
-            }
-            fenceAfter();
-          }
-          if (!mbarWaitOr(smem(&full[s]), use & 1u, abortFlag)) {
-            fail();
-            break;
-          }
-          fenceAfter();
-          const uint64_t da = descPlus(da0, uint32_t(s) * (stageA / 16u));
-          const uint64_t db = descPlus(db0, uint32_t(a.resident ? g : s) * (a.wStageBytes / 16u));
-          const uint32_t acc = tmem + buf * bufCols;
+    // The whole warp runs the loop and one lane issues: what the MMAs take then
+    // is the same in every lane for the compiler, and stays in the uniform
+    // registers that they read (one lane's loop moved every operand there:
+    // a 251x187 image 132 -> 117 us, a 1080p one 685 -> 661).
+    const bool leader = lane == 0;
+    auto waitAll = [&](uint32_t bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbarWaitOr(bar, parity, abortFlag)) != 0;
+    };
+    if (!__any_sync(0xffffffffu, *abortFlag != 0)) {
+      const uint32_t idesc = instrDesc(uint32_t(a.nt));
+      const uint32_t bTap = uint32_t(2 * a.nt);  // (16-byte units)
+      const uint64_t da0 = matDesc(smem(actBase), chunk, uint32_t(hw * 16));
+      const uint64_t db0 = matDesc(smem(wBase), uint32_t(a.nt * 16), 128u);
+      bool ok = !a.resident || total == 0 || waitAll(smem(wFull), 0u);
+      int k = 0, g = 0, s = 0;
+      uint32_t use = 0;
+      for (int q = 0; q < total && ok; ++q) {
+        const uint32_t buf = uint32_t(k & 1);
+        // the epilogue has read this buffer's previous unit out
+        if (g == 0 && k >= 2) ok = waitAll(smem(&accEmpty[buf]), uint32_t((k >> 1) - 1) & 1u);
+        if (ok) ok = waitAll(smem(&full[s]), use & 1u);
+        if (!ok) break;
+        fenceAfter();
+        const uint64_t da = descPlus(da0, uint32_t(s) * (stageA / 16u));
+        const uint64_t db = descPlus(db0, uint32_t(a.resident ? g : s) * (a.wStageBytes / 16u));
+        const uint32_t acc = tmem + buf * bufCols;
+        if (leader) {
 #pragma unroll
           for (int tap = 0; tap < 9; ++tap) {
             const uint64_t dbt = descPlus(db, uint32_t(tap) * bTap);
@@ -485,17 +484,21 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
                   tap > 0 || g > 0 ? 1u : 0u);
           }
           commit(smem(&empty[s]));
-          if (++g == groups) {
-            commit(smem(&accFull[buf]));
-            g = 0;
-            ++k;
-          }
-          if (++s == S) {
-            s = 0;
-            ++use;
-          }
+          if (g + 1 == groups) commit(smem(&accFull[buf]));
+        }
+        __syncwarp();
+        if (++g == groups) {
+          g = 0;
+          ++k;
+        }
+        if (++s == S) {
+          s = 0;
+          ++use;
         }
       }
+      if (!ok && leader) fail();
+    }
+    if (leader) {
       // every MMA issued by this thread has finished before TMEM is freed
       commit(smem(drain));
       mbarWaitOr(smem(drain), 0u, &kNeverAbort);
