@@ -28,37 +28,49 @@ constexpr uint32_t kCoreClasses = 1u << kClsTerminal | 1u << kClsLambertian | 1u
                                   1u << kClsDielectric;
 constexpr uint32_t kAllClasses = (1u << kNumShadeClasses) - 1u;
 
-// Traces the queue's ray `idx` of every lane with `active`.
-template <bool ANY>
-__device__ __forceinline__ void traceLanes(const KParams& P, const Pass& pass, bool active, uint32_t idx, int nodeLanes,
-                                           uint2* sh, uint2* loc, bool& ovf) {
-  QueueSrc<ANY, true> src;
-  src.W = &P.W;
-  src.P = &P;
-  src.fetchCtr = nullptr;
-  src.count = src.warps = 0u;
-  src.wave = pass.wave;
-  src.rO = ANY ? P.W.shO : P.W.rayO[pass.cur];
-  src.rD = ANY ? P.W.shD : P.W.rayD[pass.cur];
-  Trav<kPathThreads, kPathStack> tr;
-  tr.gMask = tr.tMask = 0u;
-  tr.bottom = 0;
-  if (active) src.load(P.S, idx, tr);
-  uint32_t events = 0, a = 0, b = 0;
-  for (;;) {
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (!act) break;
-    bool stop = false;
-    const bool done = traceRound<ANY, false>(P.S, src, tr, idx, active, act, nodeLanes, false, P.stackLimit, events, sh,
-                                             loc, a, b, ovf, stop);
-    if (stop) break;
-    if (done) {
-      active = false;
-      events = 0;
-      src.finish(idx, tr.found);
-    }
+// The ray that a lane is tracing: its path's closest hit or occlusion ray, in
+// the queue slot that the lane took.  The running kernel writes both.
+struct PathSrc {
+  QueueSrc<false, true> hit;
+  QueueSrc<true, true> shadow;
+  bool any;
+  __device__ __forceinline__ bool stopAtHit() const { return any; }
+  __device__ __forceinline__ float tmin(uint32_t i) const { return any ? shadow.tmin(i) : hit.tmin(i); }
+  template <class T>
+  __device__ __forceinline__ void load(const SceneDev& S, uint32_t i, T& tr) {
+    if (any)
+      shadow.load(S, i, tr);
+    else
+      hit.load(S, i, tr);
   }
-}
+  __device__ __forceinline__ void world(uint32_t i, float3& o, float3& d) const {
+    if (any)
+      shadow.world(i, o, d);
+    else
+      hit.world(i, o, d);
+  }
+  __device__ __forceinline__ void store(uint32_t i, float t, float u, float v, uint32_t prim, uint32_t inst) {
+    hit.store(i, t, u, v, prim, inst);
+  }
+  __device__ __forceinline__ bool later(uint32_t i, uint32_t inst, uint32_t prim) const {
+    return hit.later(i, inst, prim);
+  }
+  __device__ __forceinline__ void finish(uint32_t i, bool found) {
+    if (any)
+      shadow.finish(i, found);
+    else
+      hit.finish(i, found);
+  }
+};
+
+// What a lane's path is doing.  After shading, each lane traces its occlusion
+// ray and then its next closest hit without waiting for the others in between
+// (separate rounds for the two kinds: 32x32 box of 2 frames 172 -> 143 us, sky
+// 641x427 0.91 -> 0.83 ms, 1280x720 frame of 2.6M triangles 2.14 -> 1.94 ms).
+// Lanes that have their hit do wait for the last one: shading part of a warp
+// at a time costs more than it hides (once seven of eight wait: 0.90 and 2.06
+// ms, half of them: 1.04 and 2.33 ms).
+enum PathState : int { kPathNone, kPathHit, kPathShadow, kPathShade };
 
 template <uint32_t MASK>
 __device__ __forceinline__ void shadeAny(const KParams& P, const Pass& pass, uint32_t i, ShadeOut& out) {
@@ -100,26 +112,70 @@ __global__ void __launch_bounds__(kPathThreads, kPathMinBlocks)
     const uint32_t warps = gridDim.x * (kPathThreads / 32), warp = blockIdx.x * (kPathThreads / 32) + threadIdx.x / 32u;
     const uint32_t use = min(32u, (n + warps - 1u) / warps);
     const int nodeLanes = int(use) * kNodeLanes / 32;
-    uint32_t extends = 0, shadows = 0;
-    bool ovf = false;
-    for (uint32_t base = warp * use; base < n; base += warps * use) {
-      const uint32_t i = base + lane;
-      bool alive = lane < use && i < n;
-      for (pass.wave = from; pass.wave <= lastPass && __any_sync(0xffffffffu, alive); ++pass.wave) {
-        traceLanes<false>(P, pass, alive, i, nodeLanes, sh, lstack, ovf);
-        ShadeOut out;
-        if (alive) {
-          ++extends;
+    uint32_t extends = 0, shadows = 0, events = 0, nn = 0, nt = 0;
+    bool ovf = false, more = false, stop = false;
+    PathSrc src;
+    src.hit.W = src.shadow.W = &P.W;
+    src.hit.P = src.shadow.P = &P;
+    src.hit.rO = P.W.rayO[pass.cur];
+    src.hit.rD = P.W.rayD[pass.cur];
+    src.shadow.rO = P.W.shO;
+    src.shadow.rD = P.W.shD;
+    src.any = false;
+    Trav<kPathThreads, kPathStack> tr;
+    tr.gMask = tr.tMask = 0u;
+    tr.bottom = 0;
+    uint32_t i = warp * use + lane;
+    int state = lane < use && i < n && from <= lastPass ? kPathHit : kPathNone;
+    if (state == kPathHit) src.load(P.S, i, tr);
+    while (!stop) {
+      const unsigned tracing = __ballot_sync(0xffffffffu, state == kPathHit || state == kPathShadow);
+      const unsigned waiting = __ballot_sync(0xffffffffu, state == kPathShade);
+      if (!(tracing | waiting)) break;
+      bool next = false;  // the path's next closest hit, or the next path
+      if (!tracing) {
+        if (state == kPathShade) {
+          ShadeOut out;
           shadeAny<MASK>(P, pass, i, out);
+          ++extends;
+          if (out.next) storeNext(W, pass.cur, i, out);
+          more = out.next && pass.wave < lastPass;
+          next = !out.shadow;
+          if (out.shadow) {
+            ++shadows;
+            storeShadow(W, i, out);
+            state = kPathShadow;
+            src.any = true;
+            src.shadow.wave = pass.wave;
+            events = 0;
+            src.load(P.S, i, tr);
+          }
         }
         __syncwarp();
-        if (out.shadow) {
-          ++shadows;
-          storeShadow(W, i, out);
+      } else {
+        const bool on = tracing >> lane & 1u;
+        if (traceRound<false, false>(P.S, src, tr, i, on, tracing, nodeLanes, false, P.stackLimit, events, sh, lstack,
+                                     nn, nt, ovf, stop)) {
+          src.finish(i, tr.found);
+          next = state == kPathShadow;
+          state = kPathShade;
         }
-        if (out.next) storeNext(W, pass.cur, i, out);
-        traceLanes<true>(P, pass, out.shadow, i, nodeLanes, sh, lstack, ovf);
-        alive = out.next;
+      }
+      if (next) {
+        if (more) {
+          ++pass.wave;
+        } else {
+          i += warps * use;
+          pass.wave = from;
+        }
+        more = more || i < n;
+        state = more ? kPathHit : kPathNone;
+        if (more) {
+          src.any = false;
+          events = 0;
+          src.load(P.S, i, tr);
+        }
+        more = false;
       }
     }
     if (ovf) atomicAdd(&W.cnt->stackOverflow, 1ull);
@@ -153,7 +209,10 @@ void launchPath(const KParams& P, int lastPass, uint32_t most, int grid, cudaGra
 // (box), 0.73 / 0.19 (2M triangles); 65,536 paths 0.61 / 0.43, 1.27 / 0.68;
 // 131,072 paths 0.67 / 0.77, 1.35 / 1.03.  With the other materials, whose code
 // serialises a warp and fills the registers: 4,096 paths 2.0 / 0.58, 16,384
-// 2.2 / 1.5, 32,768 2.3 / 2.3.
+// 2.2 / 1.5, 32,768 2.3 / 2.3.  (Before a lane's occlusion ray and next closest
+// hit were traced without a wait in between, 5 to 17% less for the path kernel;
+// 65,536, 131,072 and 196,608 measured again since: within 1% at 720p, 19.5,
+// 20.0 and 21.3 ms against 19.7 for 1920x1080 of 8 frames.)
 uint32_t pathMost(uint32_t classMask) { return classMask & ~kCoreClasses ? 24576u : 98304u; }
 int pathBlocksPerSm() {
   int n = 0;

@@ -68,6 +68,7 @@ struct ArraySrc {
   int anyHit;
   static constexpr uint32_t warps = 1u;  // each warp has its own slice
   __device__ __forceinline__ uint32_t fetch(uint32_t) { return cursor; }
+  __device__ __forceinline__ bool stopAtHit() const { return false; }
   // every lane of the warp advances its copy of the cursor alike
   __device__ __forceinline__ void commit(uint32_t base, uint32_t n) { cursor = base + n; }
   template <class T>

@@ -375,7 +375,7 @@ struct Trav {
       if (COUNT) ++nTris;
       float t, b1, b2;
       if (wtTri(wt, o, p0, p1, p2, tmin, best, t, b1, b2)) {
-        if (ANY) {
+        if (ANY || src.stopAtHit()) {
           found = true;
           return true;
         }
@@ -573,6 +573,7 @@ struct QueueSrc {
   uint32_t count, warps;
   uint32_t wave;  // wavefront pass (1-based)
   __device__ __forceinline__ uint32_t fetch(uint32_t n) { return atomicAdd(fetchCtr, n); }
+  __device__ __forceinline__ bool stopAtHit() const { return ANY; }
   __device__ __forceinline__ void commit(uint32_t, uint32_t) {}
   template <class T>
   __device__ __forceinline__ void load(const SceneDev& S, uint32_t r, T& tr) {
