@@ -16,6 +16,8 @@
 //    bin chunks of a task's primitives into shared memory and merge into the
 //    task's global bins; one warp per task picks the split; blocks partition
 //    their chunks into the other order buffer (one reservation per block);
+//    the children that are large become the next level's tasks and chunks
+//    there and then, so the host waits for no level;
 //  * small tasks: one warp builds a task's whole subtree depth first with its
 //    bins and task stack in shared memory, allocating nodes from 16-node
 //    chunks so a subtree's nodes stay together; parts of at most 32

@@ -13,8 +13,9 @@
  * pooling; decoder level l: nearest x2 upsampling, concatenation with the
  * encoder output of level l, two 3x3 conv + ReLU; a 3x3 head gives a residual
  * added to log1p(radiance).  Input channels (padded to 16): log1p(radiance),
- * albedo, normal, log2(1 + filter-weight sum) / 16.  Activations NHWC bf16; images are padded to multiples of
- * 2^(L-1) internally.
+ * albedo, normal, log2(1 + filter-weight sum) / 16.  Activations bf16, in
+ * planes of eight channels; images are padded to multiples of 2^(L-1)
+ * internally.
  *
  * Parameter layout (asuna_denoiser_get_params / set_params / get_grads): for
  * each convolution in order (encoder 0..L-1 conv1, conv2; decoder L-2..0
