@@ -106,8 +106,12 @@ __global__ void __launch_bounds__(kPathThreads, kPathMinBlocks)
   Pass pass = passOf(P);
   if (handle) pass = Pass{pass.wave + 1u, pass.cur ^ 1};
   const uint32_t n = W.cnt->c[kCntExtend0 + pass.cur], from = pass.wave;
+  // The last block to leave rewrites the pass and the count.  Every thread has
+  // read both before this barrier, and its block's ticket is taken behind it, so
+  // the tickets (with the fences around them) order all reads before the writes.
+  __syncthreads();
   const unsigned lane = threadIdx.x & 31u;
-  const bool take = n <= most;  // (the same in every block: the queue is emptied after all have read it)
+  const bool take = n <= most;  // (the same in every block)
   if (take && n) {
     const uint32_t warps = gridDim.x * (kPathThreads / 32), warp = blockIdx.x * (kPathThreads / 32) + threadIdx.x / 32u;
     const uint32_t use = min(32u, (n + warps - 1u) / warps);
@@ -185,7 +189,10 @@ __global__ void __launch_bounds__(kPathThreads, kPathMinBlocks)
     if (lane == 0 && shadows) atomicAdd(&W.cnt->shadowRays, static_cast<unsigned long long>(shadows));
   }
   // the last block to leave empties the queue and decides how it goes on
-  if (threadIdx.x == 0 && atomicAdd(&W.cnt->c[kCntTicket], 1u) + 1u == gridDim.x) {
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&W.cnt->c[kCntTicket], 1u) + 1u == gridDim.x) {
+    __threadfence();
     W.cnt->c[kCntTicket] = 0u;
     if (take) W.cnt->c[kCntExtend0 + pass.cur] = 0u;
     if (handle) {
