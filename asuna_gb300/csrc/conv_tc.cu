@@ -377,9 +377,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
   // tensor memory) and set up beside this grid's last units.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // This grid's activations are there, and its outputs' last readers gone,
-  // once the layer before it has ended.  The producer and the epilogue wait
-  // for that before they touch either; the weights were there before (a grid
-  // launched alone waits for nothing).
+  // once the layer before it has ended.  Every role waits for that before it
+  // touches either and before its bounded waits; the weights were there before
+  // (a grid launched alone waits for nothing).
   auto waitForPrevious = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmemSlot, 0);
   const int groups = a.cin / 16;
@@ -459,7 +459,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__
       const uint32_t bTap = uint32_t(2 * a.nt);  // (16-byte units)
       const uint64_t da0 = matDesc(smem(actBase), chunk, uint32_t(hw * 16));
       const uint64_t db0 = matDesc(smem(wBase), uint32_t(a.nt * 16), 128u);
-      bool ok = !a.resident || total == 0 || waitAll(smem(wFull), 0u);
+      // The layer before may take any time, and its error counts from its end
+      // on: ahead of this warp's waits, whose bound is for this grid's copies.
+      waitForPrevious();
+      bool ok = !__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&g_tcError) != 0);
+      if (ok && a.resident && total > 0) ok = waitAll(smem(wFull), 0u);
       int k = 0, g = 0, s = 0;
       uint32_t use = 0;
       for (int q = 0; q < total && ok; ++q) {
