@@ -1213,18 +1213,23 @@ int asuna_scene_trace(asuna_ctx* c, const asuna_scene* s, const float* rays, uin
   ASUNA_CUDA_TRY(cudaMallocAsync(&dO, n * 16, c->stream));
   ASUNA_CUDA_TRY(cudaMallocAsync(&dD, n * 16, c->stream));
   ASUNA_CUDA_TRY(cudaMallocAsync(&dH, n * 16, c->stream));
-  ASUNA_CUDA_TRY(cudaMallocAsync(&dI, n * 4, c->stream));
+  ASUNA_CUDA_TRY(cudaMallocAsync(&dI, (size_t(n) + 1) * 4, c->stream));  // (last: traversals cut short)
   ASUNA_CUDA_TRY(cudaMemcpyAsync(dO, ho.data(), n * 16, cudaMemcpyHostToDevice, c->stream));
   ASUNA_CUDA_TRY(cudaMemcpyAsync(dD, hd.data(), n * 16, cudaMemcpyHostToDevice, c->stream));
-  launchTraceQuery(s->view, dO, dD, n, any_hit, dH, dI, c->stream);
+  ASUNA_CUDA_TRY(cudaMemsetAsync(dI + n, 0, 4, c->stream));
+  launchTraceQuery(s->view, dO, dD, n, any_hit, dH, dI, dI + n, c->stream);
   ASUNA_CUDA_TRY(cudaGetLastError());
+  uint32_t cut = 0;
   ASUNA_CUDA_TRY(cudaMemcpyAsync(hits, dH, n * 16, cudaMemcpyDeviceToHost, c->stream));
   ASUNA_CUDA_TRY(cudaMemcpyAsync(inst, dI, n * 4, cudaMemcpyDeviceToHost, c->stream));
+  ASUNA_CUDA_TRY(cudaMemcpyAsync(&cut, dI + n, 4, cudaMemcpyDeviceToHost, c->stream));
   cudaFreeAsync(dO, c->stream);
   cudaFreeAsync(dD, c->stream);
   cudaFreeAsync(dH, c->stream);
   cudaFreeAsync(dI, c->stream);
   ASUNA_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (cut)
+    return fail(ASUNA_ERR_TRAVERSAL, "ray query: traversals cut short on %u lanes (stack or loop bound)", cut);
   return ASUNA_OK;
 }
 

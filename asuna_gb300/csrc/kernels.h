@@ -80,8 +80,9 @@ int traceBlocksPerSm(int occupancy = kTraceMinBlocks, int blockThreads = kTraceT
                      int sharedStack = kSharedStack);
 int shadeBlocksPerSm();
 
-// Standalone ray queries (tests): rays are (o.xyz, tmin), (d.xyz, tmax).
+// Standalone ray queries (tests): rays are (o.xyz, tmin), (d.xyz, tmax).  Adds
+// the lanes with a traversal cut short to `cut`.
 void launchTraceQuery(const SceneDev& S, const float4* o, const float4* d, uint32_t n, int anyHit, float4* hit,
-                      uint32_t* inst, cudaStream_t s);
+                      uint32_t* inst, uint32_t* cut, cudaStream_t s);
 
 }  // namespace asuna

@@ -103,7 +103,7 @@ struct ArraySrc {
 };
 
 __global__ void __launch_bounds__(kTraceThreads) k_query(SceneDev S, const float4* o, const float4* d, uint32_t n,
-                                                         int anyHit, float4* hit, uint32_t* inst) {
+                                                         int anyHit, float4* hit, uint32_t* inst, uint32_t* cut) {
   constexpr int SHS = kSharedStack / 2;
   __shared__ uint2 sstack[SHS * kTraceThreads];
   uint2 lstack[kStackDepth - SHS];
@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_query(SceneDev S, const float
     traceWarp<true, false, kTraceThreads, SHS>(S, src, sh, lstack, kRefillLanes, true, kStackDepth, a, b, ovf);
   else
     traceWarp<false, false, kTraceThreads, SHS>(S, src, sh, lstack, kRefillLanes, true, kStackDepth, a, b, ovf);
+  if (ovf) atomicAdd(cut, 1u);
 }
 
 }  // namespace
@@ -185,11 +186,11 @@ int traceBlocksPerSm(int occupancy, int blockThreads, int sharedStack) {
   return n > 0 ? n : 1;
 }
 void launchTraceQuery(const SceneDev& S, const float4* o, const float4* d, uint32_t n, int anyHit, float4* hit,
-                      uint32_t* inst, cudaStream_t s) {
+                      uint32_t* inst, uint32_t* cut, cudaStream_t s) {
   int grid = int((n + kTraceThreads - 1) / kTraceThreads);
   if (grid > 4096) grid = 4096;
   if (grid < 1) grid = 1;
-  k_query<<<grid, kTraceThreads, 0, s>>>(S, o, d, n, anyHit, hit, inst);
+  k_query<<<grid, kTraceThreads, 0, s>>>(S, o, d, n, anyHit, hit, inst, cut);
 }
 
 }  // namespace asuna

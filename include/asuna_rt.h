@@ -443,7 +443,9 @@ int asuna_render_paths(asuna_ctx* ctx, const asuna_scene* scene, const asuna_sho
 
 /* Traversal query (tests, tools): n rays of 8 floats (o.xyz, tmin, d.xyz,
  * tmax); hits receive (t, u, v, primitive bits) or t = -1 on a miss, inst the
- * instance index or 0xffffffff.  any_hit = 1 gives occlusion only. */
+ * instance index or 0xffffffff.  any_hit = 1 gives occlusion only.
+ * ASUNA_ERR_TRAVERSAL if a traversal was cut short (a loop bound, as in a
+ * render): the hits of such rays may be wrong. */
 int asuna_scene_trace(asuna_ctx* ctx, const asuna_scene* scene, const float* rays, uint32_t n, int any_hit,
                       float* hits, uint32_t* inst);
 
