@@ -295,6 +295,7 @@ int buildWide(const BvhNode* nodes, uint32_t nodeCount, const TriDev* tris, uint
     return fail(ASUNA_ERR_INVALID, "wide BVH: collapse failed (error bits %u, %u of %u triangles, %u of %u instances)",
                 ctr[kWError], ctr[kWTris], triCount, ctr[kWInst], instCount);
   out.nodeCount = ctr[kWNodes];
+  while (out.levels < uint32_t(levels) && ctr[kWLevel0 + out.levels]) ++out.levels;
   if (keep) {
     out.bytes = size_t(nodeCap) * sizeof(WideNode) + triCount * sizeof(TriDev) + (size_t(instCount) + 1) * 4;
     return ASUNA_OK;

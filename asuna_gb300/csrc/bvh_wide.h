@@ -16,6 +16,7 @@ struct WideBvh {
   uint32_t* instIds = nullptr;  // device; instances in wide-leaf order of the top level (in the block of `tris`)
   size_t bytes = 0;             // of both blocks
   uint32_t nodeCount = 0;
+  uint32_t levels = 0;        // of the deepest tree
   std::vector<uint32_t> rootLeaves;  // InstDev::rootLeaves of every root
 };
 

@@ -146,6 +146,7 @@ struct SceneDev {
   float4 boundLo;        // world bounds of the instances (xyz) ...
   float4 cellScale;      // ... and 4 / extent per axis: the ray-sort origin cells
   int32_t tlasRoot;
+  int32_t treeLevels;  // levels of the deepest tree of wide nodes
   int32_t envW, envH;
   int32_t numInst;
   uint32_t classMask;  // shading classes some instance can reach (bit k = class k)

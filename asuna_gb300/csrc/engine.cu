@@ -744,6 +744,7 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
     }
   }
   v.tlasRoot = int32_t(wideRoots.size() - 1);
+  v.treeLevels = int32_t(wide.levels);
   std::memset(&v.sky, 0, sizeof(v.sky));
   if (d->sun_and_sky && d->sun_and_sky->in_use == 1) {
     v.sky = *d->sun_and_sky;

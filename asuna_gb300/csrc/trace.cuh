@@ -464,8 +464,7 @@ __device__ __forceinline__ bool traceRound(const SceneDev& S, Src& src, T& tr, u
                                            int nodeLanes, bool spec, int lim, uint32_t& events, uint2* sh, uint2* loc,
                                            uint32_t& nNodes, uint32_t& nTris, bool& ovf, bool& stop) {
   // Node steps while enough lanes want one.  Lanes with a leaf group in
-  // hand walk on when `spec` (and there is room for a second group on the
-  // stack).  A pass that stops early leaves lanes at a leaf or a
+  // hand walk on when `spec` (and there is room on the stack).  A pass that stops early leaves lanes at a leaf or a
   // transition, which go on below: some lane advances in every round.
   // Both loops carry a bound far above any real traversal: past it the
   // warp stops and reports the error instead of running on.
@@ -475,7 +474,10 @@ __device__ __forceinline__ bool traceRound(const SceneDev& S, Src& src, T& tr, u
     const unsigned wm = __ballot_sync(0xffffffffu, want);
     if (wm == 0u || (__popc(wm) < nodeLanes && wm != act)) break;
     if (++spin > kTraceSpinCap) break;
-    if (want || (spec && active && tr.hasNodes() && tr.bottom != 0 && tr.sp + 4 < lim))
+    // A speculative step pushes two entries, and the ordered steps below it one
+    // on each further level (of treeLevels - 1 at most): with room for all of
+    // them, speculation never overflows a stack that the ordered walk fits.
+    if (want || (spec && active && tr.hasNodes() && tr.bottom != 0 && tr.sp + S.treeLevels < lim))
       tr.template nodeStep<COUNT>(S, src.tmin(idx), sh, loc, lim, nNodes, ovf);
   }
   if (spin > kTraceSpinCap) {
