@@ -186,6 +186,7 @@ SIGNATURES = [
     ("asuna_render", C.c_int, [P, P, C.POINTER(Shot), P, C.POINTER(RenderStats)]),
     ("asuna_render_batch", C.c_int, [P, P, C.POINTER(Shot), C.POINTER(P), C.c_uint32, C.POINTER(RenderStats)]),
     ("asuna_render_paths", C.c_int, [P, P, C.POINTER(Shot), P, P]),
+    ("asuna_ctx_path_stats", C.c_int, [P, C.POINTER(C.c_double), C.POINTER(C.c_uint64)]),
     ("asuna_scene_trace", C.c_int, [P, P, P, C.c_uint32, C.c_int, P, P]),
     ("asuna_json_load", C.c_int, [C.c_char_p, C.POINTER(P)]),
     ("asuna_json_load_string", C.c_int, [C.c_char_p, C.c_char_p, C.POINTER(P)]),

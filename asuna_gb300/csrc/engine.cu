@@ -945,7 +945,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
   if (hostRecords) ASUNA_CUDA_TRY(cudaMallocAsync(&dRec, totalPaths * sizeof(asuna_path_record), c->stream));
   // the statistics start at zero; the cut-short count (last) is cumulative
   if (stats) ASUNA_CUDA_TRY(cudaMemsetAsync(c->cnt, 0, offsetof(DevCounters, stackOverflow), c->stream));
-  // timing events: [begin, end] + one pair per extend / shade / connect launch
+  // timing events: [begin, end] + one pair per path / sort / extend / shade / connect launch
   size_t evNeed = 2;
   for (auto& b : batches) evNeed += size_t(wavefrontPasses(b.maxDepth, s->view)) * 10;
   if (stats) {
@@ -1038,7 +1038,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     launches += 2;
     P.depth = 1;
     if (b.paths <= most) {
-      timedLaunch(0, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
+      timedLaunch(4, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
       ++launches;
     } else if (loopGraph && passes > 1) {
       // The later passes as a loop in the graph that ends when no ray is left
@@ -1083,7 +1083,7 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
       for (int depth = 2; depth <= passes; ++depth) {
         P.depth = uint32_t(depth);
         if (most) {
-          timedLaunch(0, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
+          timedLaunch(4, [&] { launchPath(P, passes, most, c->pathGrid, 0, c->stream); });
           ++launches;
         }
         if (c->raySort) {
@@ -1162,6 +1162,8 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
     float ms = 0;
     ASUNA_CUDA_TRY(cudaEventElapsedTime(&ms, c->events[0], c->events[1]));
     stats->ms_total = ms;
+    c->pathMs = 0.0;
+    c->pathLaunches = 0;
     for (auto& t : timed) {
       float m = 0;
       ASUNA_CUDA_TRY(cudaEventElapsedTime(&m, c->events[t.second], c->events[t.second + 1]));
@@ -1172,6 +1174,9 @@ static int renderImpl(asuna_ctx* c, const asuna_scene* s, const asuna_shot* shot
         stats->ms_shade += m;
       } else if (t.first == 3) {
         stats->ms_sort += m;
+      } else if (t.first == 4) {
+        c->pathMs += m;
+        c->pathLaunches++;
       } else {
         stats->ms_connect += m;
         stats->connect_launches++;
@@ -1196,6 +1201,13 @@ int asuna_render_paths(asuna_ctx* c, const asuna_scene* s, const asuna_shot* sho
                        asuna_path_record* host_records) {
   if (!host_records) return fail(ASUNA_ERR_INVALID, "null records");
   return renderImpl(c, s, shot, &film, 1, nullptr, host_records);
+}
+
+int asuna_ctx_path_stats(const asuna_ctx* c, double* ms_path, uint64_t* path_launches) {
+  if (!c || !ms_path || !path_launches) return fail(ASUNA_ERR_INVALID, "null argument");
+  *ms_path = c->pathMs;
+  *path_launches = c->pathLaunches;
+  return ASUNA_OK;
 }
 
 int asuna_scene_trace(asuna_ctx* c, const asuna_scene* s, const float* rays, uint32_t n, int any_hit, float* hits,

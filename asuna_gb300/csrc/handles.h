@@ -64,6 +64,8 @@ struct asuna_ctx {
   // as much (21M-triangle scene, ms per render sorted / unsorted: 8 frames
   // 21.9 / 21.7, 256 frames 434.7 / 434.0; a 1280x720 frame 2.23 / 2.05).
   int32_t raySort = 0;
+  double pathMs = 0.0;        // asuna_ctx_path_stats
+  uint64_t pathLaunches = 0;
   int32_t stackLimit = 0; // traversal stack entries a ray may use (0 = the compiled capacity)
   int32_t bvhBuild = 0;   // bottom-level BVHs: 0 built on the device, 1 on host threads
   // traversals cut short on the device: the cumulative device count is

@@ -561,8 +561,11 @@ class DeviceScene:
     __del__ = close
 
 
-def _stats_dict(s):
-    return {k: getattr(s, k) for k, _ in A.RenderStats._fields_}
+def _stats_dict(ctx, s):
+    ms, launches = C.c_double(), C.c_uint64()
+    check(lib().asuna_ctx_path_stats(ctx.handle, C.byref(ms), C.byref(launches)))
+    return {**{k: getattr(s, k) for k, _ in A.RenderStats._fields_}, "ms_path": ms.value,
+            "path_launches": launches.value}
 
 
 class Context:
@@ -634,7 +637,7 @@ class Context:
         st = A.RenderStats() if stats else None
         check(lib().asuna_render(self.handle, scene.handle, C.byref(shot), film.handle,
                                  C.byref(st) if st is not None else None))
-        return _stats_dict(st) if st is not None else None
+        return _stats_dict(self, st) if st is not None else None
 
     def render_batch(self, scene, shots, films, stats=False):
         n = len(shots)
@@ -642,7 +645,7 @@ class Context:
         fh = (C.c_void_p * n)(*[f.handle for f in films])
         st = A.RenderStats() if stats else None
         check(lib().asuna_render_batch(self.handle, scene.handle, sh, fh, n, C.byref(st) if st is not None else None))
-        return _stats_dict(st) if st is not None else None
+        return _stats_dict(self, st) if st is not None else None
 
     def render_paths(self, scene, shot, film):
         rec = np.zeros(shot.frames * shot.width * shot.height, A.PATH_RECORD_DTYPE)

@@ -349,7 +349,8 @@ def run(args):
         torch_dist.barrier()
     ctx.sync()
     tot = {k: 0.0 for k in ("extend_rays", "shadow_rays", "paths", "ms_total", "ms_extend", "ms_connect",
-                            "ms_shade", "ms_sort", "extend_launches", "connect_launches", "kernel_launches")}
+                            "ms_shade", "ms_sort", "ms_path", "extend_launches", "connect_launches",
+                            "kernel_launches")}
     with ClockSampler(local) as clk:
         for i in range(args.steps):
             st = step(1 + args.warmup + i)
@@ -389,6 +390,8 @@ def run(args):
             torch_dist.destroy_process_group()
         return 0
     peak, peak_kind = peaks()
+    # (the rays that the path kernel traces at the end of a wave, at most 98,304 a
+    # pass of the wave's hundreds of millions, are in extend_rays as well)
     ext_ms_per_launch = tot["ms_extend"] / max(tot["extend_launches"], 1)
     ext_bytes_per_launch = bytes_per_ext * tot["extend_rays"] / max(tot["extend_launches"], 1)
     achieved = ext_bytes_per_launch / (ext_ms_per_launch * 1e-3) / 1e9
@@ -420,7 +423,7 @@ def run(args):
                      "traffic": traffic, "bytes_per_ray": bytes_per_ext, "shadow_bytes_per_ray": bytes_per_sh,
                      "ms_per_launch": ext_ms_per_launch},
         "kernel_ms": {"extend": tot["ms_extend"], "shade": tot["ms_shade"], "connect": tot["ms_connect"],
-                      "sort": tot["ms_sort"]},
+                      "sort": tot["ms_sort"], "path": tot["ms_path"]},
         "clocks": clk.summary(),
         "scene": {"triangles": sstats["triangles"], "device_bytes": sstats["device_bytes"],
                   "build_ms": sstats["build_ms"]},

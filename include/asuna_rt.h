@@ -441,6 +441,13 @@ int asuna_render_batch(asuna_ctx* ctx, const asuna_scene* scene, const asuna_sho
 int asuna_render_paths(asuna_ctx* ctx, const asuna_scene* scene, const asuna_shot* shot,
                        asuna_film* film, asuna_path_record* host_records);
 
+/* The path kernel's part of the context's last render with stats: it traces and
+ * shades a wave of few paths, and the last rays of a larger one, in one launch.
+ * None of it is in the ms_extend, ms_connect, ms_shade and *_launches of
+ * asuna_render_stats (a wave that it takes whole leaves those at 0); its rays
+ * are in extend_rays and shadow_rays, its launches in kernel_launches. */
+int asuna_ctx_path_stats(const asuna_ctx* ctx, double* ms_path, uint64_t* path_launches);
+
 /* Traversal query (tests, tools): n rays of 8 floats (o.xyz, tmin, d.xyz,
  * tmax); hits receive (t, u, v, primitive bits) or t = -1 on a miss, inst the
  * instance index or 0xffffffff.  any_hit = 1 gives occlusion only.
