@@ -177,6 +177,7 @@ SIGNATURES = [
     ("asuna_sun_and_sky_default", None, [C.POINTER(SunAndSky)]),
     ("asuna_scene_validate", C.c_int, [C.POINTER(SceneDesc)]),
     ("asuna_scene_destroy", C.c_int, [P]),
+    ("asuna_scene_envmap_tables", C.c_int, [P, P, P]),
     ("asuna_scene_get_stats", C.c_int, [P, C.POINTER(SceneStats)]),
     ("asuna_film_create", C.c_int, [P, C.c_uint32, C.c_uint32, C.POINTER(P)]),
     ("asuna_film_destroy", C.c_int, [P]),

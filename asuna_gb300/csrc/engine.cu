@@ -770,6 +770,16 @@ int asuna_scene_destroy(asuna_scene* s) {
   return ASUNA_OK;
 }
 
+int asuna_scene_envmap_tables(const asuna_scene* s, float* marginal, float* conditional) {
+  clearError();
+  if (!s || !marginal || !conditional) return fail(ASUNA_ERR_INVALID, "null argument");
+  ASUNA_CUDA_TRY(cudaSetDevice(s->device));
+  const size_t bytes = size_t(s->view.envW) * size_t(s->view.envH) * sizeof(float2);
+  ASUNA_CUDA_TRY(cudaMemcpy(marginal, s->view.marg, bytes, cudaMemcpyDeviceToHost));
+  ASUNA_CUDA_TRY(cudaMemcpy(conditional, s->view.cond, bytes, cudaMemcpyDeviceToHost));
+  return ASUNA_OK;
+}
+
 int asuna_scene_get_stats(const asuna_scene* s, asuna_scene_stats* out) {
   if (!s || !out) return fail(ASUNA_ERR_INVALID, "null argument");
   *out = s->stats;

@@ -540,6 +540,13 @@ class DeviceScene:
         check(lib().asuna_scene_get_stats(self.handle, C.byref(s)))
         return {k: getattr(s, k) for k, _ in A.SceneStats._fields_}
 
+    def envmap_tables(self, width, height):
+        """The importance tables of the scene's width x height environment map as
+        the device holds them (laid out as the module's envmap_tables)."""
+        marg, cond = np.empty((height, width, 2), np.float32), np.empty((height, width, 2), np.float32)
+        check(lib().asuna_scene_envmap_tables(self.handle, marg.ctypes.data, cond.ctypes.data))
+        return marg, cond
+
     def trace(self, origins, dirs, tmin=1e-5, tmax=1e10, any_hit=False):
         n = len(origins)
         rays = np.zeros((n, 8), np.float32)

@@ -409,6 +409,9 @@ int asuna_scene_create(asuna_ctx* ctx, const asuna_scene_desc* desc, asuna_scene
 void asuna_sun_and_sky_default(asuna_sun_and_sky* out);
 int asuna_scene_destroy(asuna_scene* scene);
 int asuna_scene_get_stats(const asuna_scene* scene, asuna_scene_stats* out);
+/* The environment map's importance tables as the device holds them (tests,
+ * tools), laid out as asuna_envmap_tables fills them; 1 x 1 without a map. */
+int asuna_scene_envmap_tables(const asuna_scene* scene, float* marginal_xy, float* conditional_xy);
 /* The checks asuna_scene_create runs before any upload (indices in range,
  * implemented material types and features, lights), on the host alone. */
 int asuna_scene_validate(const asuna_scene_desc* desc);
