@@ -21,9 +21,9 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA, "bin", "nvcc") if os.path.exists(os.path.join(CUDA, "bin", "nvcc")) else "nvcc"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU = {"trace.cu": [], "shade.cu": ["-fmad=false"], "path.cu": ["-fmad=false"], "env_tables.cu": ["-fmad=false"], "engine.cu": [], "noalloc.cu": [], "denoise.cu": [], "post.cu": [],
-      "conv_tc.cu": [], "queue_sort.cu": [], "mesh_upload.cu": [], "bvh_device.cu": ["-fmad=false"],
-      "bvh_wide.cu": []}
+CU = {"trace.cu": [], "shade.cu": ["-fmad=false"], "path.cu": ["-fmad=false"], "env_tables.cu": ["-fmad=false"],
+      "engine.cu": [], "noalloc.cu": [], "denoise.cu": [], "post.cu": [], "conv_tc.cu": [], "queue_sort.cu": [],
+      "mesh_upload.cu": [], "bvh_device.cu": ["-fmad=false"], "bvh_wide.cu": []}
 CPP = ["host_scene.cpp", "json.cpp", "bvh_build.cpp", "server.cpp"]
 
 

@@ -114,7 +114,7 @@ namespace {
 // Pixel tiles per unit (T), resident CTAs per SM, ring depth and weight
 // residency: the choice with the most tiles in flight per SM (T x CTAs),
 // where a CTA needs two accumulator buffers of T x nt tensor-memory columns
-// (512 per SM), its shared memory, and 192 threads of 72 registers (four
+// (512 per SM), its shared memory, and 192 threads of at most 80 registers (four
 // CTAs fit); then resident weights (single-slice layers whose weights fit:
 // read from L2 once per CTA instead of once per unit), then the deepest ring
 // the CTAs' shared memory holds; ties go to smaller T (more CTAs, rings that
@@ -329,8 +329,8 @@ constexpr int kThreads = 32 * (kEpiWarps + 2);
 template <int T>
 __global__ void __launch_bounds__(kThreads, 4) k_conv_tc(const __grid_constant__ CUtensorMap act, TcArgs a) {
   extern __shared__ __align__(1024) unsigned char sm[];
-  // [0, 128): barriers, the TMEM address and the abort flag; then the
-  // activation stages and the weight stages
+  // [0, kBarriers): barriers, the TMEM address and the abort flag; then the
+  // epilogue warps' bias, the activation stages and the weight stages
   uint64_t* full = reinterpret_cast<uint64_t*>(sm);
   uint64_t* empty = full + kMaxStages;
   uint64_t* accFull = empty + kMaxStages;

@@ -63,7 +63,7 @@ constexpr int kWideExpBias = 127 + 15;      // the traversal wants the float 2^(
 constexpr int kWideMaxExp = 254 - kWideExpBias;
 constexpr float kWideFar = 1e34f;           // box planes beyond this (or NaN) are moved here
 
-constexpr int kMaxLeafTris = 8;
+constexpr int kMaxLeafTris = 8;  // what a leaf reference can count
 constexpr int32_t kStackSentinel = INT32_MIN;  // "leave the BLAS" marker
 inline __host__ __device__ int32_t encodeLeaf(uint32_t first, uint32_t count) {
   return ~int32_t(first * 8u + (count - 1u));

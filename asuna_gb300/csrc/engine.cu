@@ -378,7 +378,7 @@ int asuna_scene_create(asuna_ctx* c, const asuna_scene_desc* d, asuna_scene** ou
   s->device = c->device;
   std::unique_ptr<asuna_scene, int (*)(asuna_scene*)> guard(s, asuna_scene_destroy);
 
-  // ---- bottom level: one BVH per mesh, built on host threads ----
+  // ---- meshes: vertices and indices in one array each ----
   const uint32_t nm = d->num_meshes;
   std::vector<uint32_t> triBase(nm + 1, 0), vtxBase(nm + 1, 0);
   for (uint32_t m = 0; m < nm; ++m) {

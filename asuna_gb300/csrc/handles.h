@@ -54,15 +54,11 @@ struct asuna_ctx {
   int32_t occupancy = 8;  // traversal kernel variant: resident 128-thread blocks per SM (8, 10, 12)
   int32_t occupancyShadow = 8;  // the same for the occlusion pass
   int32_t traceThreads = 128;  // traversal kernel variant: threads per block
-  int32_t sharedStack = 24;    // traversal kernel variant: stack entries in shared memory
+  int32_t sharedStack = 24;    // traversal kernel variant: stack words in shared memory, two an entry
   // extend-queue sort mode before secondary passes (0 off).  Off by default:
-  // with the 8-wide nodes the sort gains the extend pass 5% at most and costs
-  // as much (21M-triangle scene, ms per render sorted / unsorted: 8 frames
-  // 19.2 / 18.8, 256 frames 434.7 / 434.0; a 320x180 preview 1.29 / 1.13).
-  // extend-queue sort mode before secondary passes (0 off).  Off by default:
-  // with the 8-wide nodes the sort gains the extend pass 5% at most and costs
-  // as much (21M-triangle scene, ms per render sorted / unsorted: 8 frames
-  // 21.9 / 21.7, 256 frames 434.7 / 434.0; a 1280x720 frame 2.23 / 2.05).
+  // with the 8-wide nodes the sort gains the extend pass 6% at most and costs
+  // nearly as much (ms per render sorted / unsorted, 1920x1080 of 21M triangles:
+  // 8 frames 19.2 / 18.9, 256 frames 465.3 / 467.5; a 1280x720 frame 2.15 / 2.00).
   int32_t raySort = 0;
   double pathMs = 0.0;        // asuna_ctx_path_stats
   uint64_t pathLaunches = 0;

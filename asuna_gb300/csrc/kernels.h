@@ -18,7 +18,7 @@ struct KParams {
   int32_t occupancy;     // traversal: resident blocks per SM of the kernel variant (8, 10 or 12)
   int32_t stackLimit;    // traversal: stack entries a ray may use, in [1, kStackDepth] (the host clamps it)
   int32_t blockThreads;  // traversal: threads per block (64, 128, 256; 0 = 128)
-  int32_t sharedStack;   // traversal: stack entries in shared memory (16, 24, 32; 0 = 24)
+  int32_t sharedStack;   // traversal: stack words in shared memory (16, 24, 32; 0 = 24), two an entry
 };
 
 // The wavefront pass that a kernel works on.  A pass that a graph repeats
@@ -37,7 +37,7 @@ __device__ __forceinline__ Pass passOf(const KParams& P) {
 constexpr int kTraceThreads = 128;
 constexpr int kTraceMinBlocks = 8;   // resident blocks per SM the traversal kernels are compiled for
 constexpr int kStackDepth = 64;      // traversal stack entries per ray
-constexpr int kSharedStack = 24;     // of which in shared memory (the rest in local memory)
+constexpr int kSharedStack = 24;     // words in shared memory, two an entry (the rest in local memory)
 constexpr int kRefillLanes = 8;      // default idle lanes of a warp that trigger a queue fetch
 constexpr int kShadeMinBlocks = 3;   // resident 256-thread blocks per SM the shading kernel is compiled for
 
@@ -75,7 +75,7 @@ uint32_t pathMost(uint32_t classMask);
 int pathBlocksPerSm();
 void launchConnect(const KParams& P, int grid, cudaStream_t s);
 // resident blocks per SM of the traversal variant (occupancy class 8/10/12 =
-// 32/40/48 resident warps, block size, shared-memory stack entries)
+// 32/40/48 resident warps, block size, shared-memory stack words)
 int traceBlocksPerSm(int occupancy = kTraceMinBlocks, int blockThreads = kTraceThreads,
                      int sharedStack = kSharedStack);
 int shadeBlocksPerSm();

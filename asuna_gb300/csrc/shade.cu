@@ -145,7 +145,6 @@ __global__ void __launch_bounds__(256) k_raygen(KParams P) {
 }
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Splits the hits of the extend queue into the shading classes (material
 // sort).  A block takes 256 hits at a time: lanes are grouped by class in
 // each warp (one shared-memory add per class present), then one global

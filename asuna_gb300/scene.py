@@ -615,8 +615,8 @@ class Context:
 
     def set_traversal_shape(self, threads_per_block=0, shared_stack=0):
         """Traversal kernel variant: threads per block (64, 128, 256) and
-        stack entries in shared memory (16, 24, 32); 0 = defaults.  Results
-        do not depend on them."""
+        32-bit stack words in shared memory (16, 24, 32; two an entry); 0 =
+        defaults.  Results do not depend on them."""
         check(lib().asuna_ctx_set_traversal_shape(self.handle, int(threads_per_block), int(shared_stack)))
 
     def set_traversal_occupancy(self, extend_blocks_per_sm=0, shadow_blocks_per_sm=0):

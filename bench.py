@@ -48,7 +48,7 @@ METRIC = "Mrays/s"
 CONFIG = {"workload": "mixed-material scene, 64 x level-7 icospheres (20.97M tris), 1920x1080, depth 12, RR>3, "
                       "1024x512 env + 4 triangle lights, aperture 0.05",
           "triangles": 20971526, "width": 1920, "height": 1080, "max_depth": 12, "rr_depth": 3,
-          "l2": "inputs larger than L2 (BVH ~2.7 GB), no flush"}
+          "l2": "inputs larger than L2 (BVH 1.2 GB), no flush"}
 
 
 def dist_env():
@@ -678,7 +678,7 @@ def run_denoise_forward(args):
     tc = res["tcgen05"]
     print(json.dumps({"metric": "denoiser forward TFLOP/s", "value": tc["tflops"], "unit": "TFLOP/s",
                       "higher_is_better": True, "steps": args.steps, "warmup": args.warmup, "ms_per_step": tc["ms"],
-                      "config": {"workload": f"U-Net 32/48/64/96/128, 1 x {hp} x {wp}, bf16 NHWC, fp32 accumulation",
+                      "config": {"workload": f"U-Net 32/48/64/96/128, 1 x {hp} x {wp}, bf16 in planes of 8 channels, fp32 accumulation",
                                  "flop": fl},
                       "roofline": {"bound": "tensor", "achieved": tc["tflops"], "peak": peak, "unit": "TFLOP/s",
                                    "frac": tc["tflops"] / peak, "peak_kind": kind},

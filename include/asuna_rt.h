@@ -331,9 +331,9 @@ typedef struct asuna_render_stats {
 typedef struct asuna_scene_stats {
   uint64_t triangles;
   uint64_t instances;
-  uint64_t blas_nodes;
-  uint64_t tlas_nodes;
-  uint64_t device_bytes;
+  uint64_t blas_nodes;   /* nodes of the binary trees that the builders made ... */
+  uint64_t tlas_nodes;   /* ... which the scene keeps as fewer, 8-wide nodes */
+  uint64_t device_bytes; /* held by the scene */
   double build_ms;
 } asuna_scene_stats;
 
@@ -375,9 +375,9 @@ int asuna_ctx_set_launch(asuna_ctx* ctx, int trace_blocks_per_sm, int shade_bloc
 int asuna_ctx_set_traversal(asuna_ctx* ctx, int refill_extend, int refill_shadow, int speculate_extend,
                             int speculate_shadow, int blocks_per_sm);
 /* Shape of the traversal kernel variant: threads per block (64, 128 or 256)
- * and traversal-stack entries kept in shared memory (16, 24 or 32; the rest
- * of the 64 in thread-local memory); 0 = 128 / 24.  Results do not depend
- * on them. */
+ * and 32-bit words of the traversal stack kept in shared memory (16, 24 or 32:
+ * 8, 12 or 16 entries; the rest of the 64 in thread-local memory); 0 = 128 /
+ * 24.  Results do not depend on them. */
 int asuna_ctx_set_traversal_shape(asuna_ctx* ctx, int threads_per_block, int shared_stack_entries);
 /* The traversal kernel variant's resident blocks per SM of the closest-hit
  * (extend) and occlusion (shadow) passes separately (8, 10 or 12; 0 = 8);
